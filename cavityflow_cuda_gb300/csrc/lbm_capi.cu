@@ -230,12 +230,62 @@ int step(lbm_solver* s, bool alpha, const int32_t* origin, const int32_t* size, 
     return LBM_OK;
 }
 
+void drop_pairs(lbm_solver* s)
+{
+    if (!s->dd2) return;
+    cudaFree(s->dd2);
+    s->dd2 = nullptr;
+    s->device_bytes -= (int64_t)((size_t)lbm::Q * s->g.S * elem_bytes(s->storage));
+}
+
+// cudaMalloc that gives up lbm_run's second population array rather than fail.
+cudaError_t alloc_or_drop_pairs(lbm_solver* s, void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && s->dd2) {
+        cudaGetLastError();
+        drop_pairs(s);
+        s->pairs_refused = true;
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+// Whether lbm_run takes two steps a pass on `st` (launch_pair_step, between dd
+// and dd2 and back, so that the state is always in dd when a call returns).
+// The second array is allocated on first use, and only while it is at most a
+// quarter of the free memory, so that a solver which fills the card keeps what
+// it could do without it.  A capturing stream gets the separate kernels: the
+// caller's graph must not hold an array that the solver may give up.
+bool ensure_pairs(lbm_solver* s, cudaStream_t st)
+{
+    if (!s->pairs || s->pairs_refused || s->fma || s->lid_y < 0 || !s->owns_dd) return false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (capture != cudaStreamCaptureStatusNone || !lbm::pair_step_pays(s->storage, s->g)) return false;
+    if (s->dd2) return true;
+    const size_t bytes = (size_t)lbm::Q * s->g.S * elem_bytes(s->storage);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 ||
+        cudaMalloc(&s->dd2, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        s->dd2 = nullptr;
+        s->pairs_refused = true;
+        return false;
+    }
+    s->device_bytes += (int64_t)bytes;
+    return true;
+}
+
 int ensure_macros(lbm_solver* s)
 {
     CK(cudaSetDevice(s->device), "cudaSetDevice");
     if (!s->macros) {
         const size_t bytes = (size_t)4 * s->g.cells() * value_bytes(s->storage);
-        CK(cudaMalloc(&s->macros, bytes), "cudaMalloc macros");
+        CK(alloc_or_drop_pairs(s, &s->macros, bytes), "cudaMalloc macros");
         s->device_bytes += (int64_t)bytes;
         s->macros_fresh = false;
     }
@@ -300,7 +350,7 @@ int ensure_staging(lbm_solver* s, size_t elems)
         s->staging = nullptr;
         s->staging_elems = 0;
     }
-    CK(cudaMalloc(&s->staging, elems * sizeof(float)), "cudaMalloc staging");
+    CK(alloc_or_drop_pairs(s, (void**)&s->staging, elems * sizeof(float)), "cudaMalloc staging");
     s->staging_elems = elems;
     s->device_bytes += (int64_t)(elems * sizeof(float));
     return LBM_OK;
@@ -471,6 +521,7 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
                     lbm::kFastVariantCount);
     }
     s->variant = prm->fast_variant == 0 ? default_variant(s->storage) : prm->fast_variant - 1;
+    s->pairs = prm->fast_variant == 0;
     s->fma = prm->fused_multiply_add == 1;
     s->lid_mode = prm->lid_mode;
 
@@ -522,6 +573,7 @@ void lbm_detail::destroy_solver(lbm_solver* s)
     drop_graph(s);
     if (s->capture_stream) cudaStreamDestroy(s->capture_stream);
     if (s->dd && s->owns_dd) cudaFree(s->dd);
+    if (s->dd2) cudaFree(s->dd2);
     if (s->flags) cudaFree(s->flags);
     if (s->macros) cudaFree(s->macros);
     if (s->scratch) cudaFree(s->scratch);
@@ -645,6 +697,23 @@ int lbm_run(lbm_solver* s, int64_t steps, void* stream)
         if (int r = step(s, false, nullptr, nullptr, st)) return r;
         --left;
     }
+    // pairs there and back: the kernels are long enough to need no graph
+    if (steps >= 2 && ensure_pairs(s, st)) {
+        int* const work = reinterpret_cast<int*>(s->counts + 3);
+        lbm::Params p = s->p;
+        p.step_base = step_words(s) + 1;
+        for (; left >= 4; left -= 4) {
+            p.step_off = (uint32_t)s->counter;
+            CK(lbm::launch_pair_step(s->storage, s->dd, s->dd2, s->g, p, s->lid_y, work, err_flag(s), st),
+               "pair step launch");
+            p.step_off = (uint32_t)(s->counter + 2);
+            CK(lbm::launch_pair_step(s->storage, s->dd2, s->dd, s->g, p, s->lid_y, work, err_flag(s), st),
+               "pair step launch");
+            s->counter += 4;
+            s->last_alpha = false;
+            s->macros_fresh = false;
+        }
+    }
     const int64_t per_graph = 2 * kGraphPairs;
     if (s->lid_y >= 0 && left >= per_graph) {
         if (!s->graph) {
@@ -716,9 +785,8 @@ int lbm_selftest_bounded_wait(lbm_solver* s, int32_t limit_us)
 int lbm_fast_variant_count(void) { return lbm::kFastVariantCount; }
 int lbm_register_variant_count(void) { return lbm::kRegisterVariants; }
 
-int lbm_set_fast_variant(lbm_solver* s, int32_t variant)
+static int select_variant(lbm_solver* s, int32_t variant)
 {
-    if (int r = check_solver(s)) return r;
     if (variant < 0 || variant >= lbm::kFastVariantCount)
         return fail(LBM_ERR_INVALID_ARGUMENT, "variant %d not in [0, %d)", variant, lbm::kFastVariantCount);
     CK(cudaSetDevice(s->device), "cudaSetDevice");
@@ -726,6 +794,14 @@ int lbm_set_fast_variant(lbm_solver* s, int32_t variant)
         return fail(LBM_ERR_UNSUPPORTED, "variant %d needs more shared memory than this domain allows", variant);
     if (variant != s->variant) drop_graph(s);
     s->variant = variant;
+    return LBM_OK;
+}
+
+int lbm_set_fast_variant(lbm_solver* s, int32_t variant)
+{
+    if (int r = check_solver(s)) return r;
+    if (int r = select_variant(s, variant)) return r;
+    s->pairs = false;  // every step with the variant asked for
     return LBM_OK;
 }
 
@@ -738,7 +814,7 @@ int lbm_autotune(lbm_solver* s, int32_t pairs, int32_t* best, float* ms_per_pair
     CK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     const size_t bytes = (size_t)lbm::Q * s->g.S * elem_bytes(s->storage);
     void* saved = nullptr;
-    CK(cudaMalloc(&saved, bytes), "cudaMalloc autotune snapshot");
+    CK(alloc_or_drop_pairs(s, &saved, bytes), "cudaMalloc autotune snapshot");
     cudaStream_t st = s->capture_stream;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int result = LBM_OK;
@@ -791,7 +867,7 @@ int lbm_autotune(lbm_solver* s, int32_t pairs, int32_t* best, float* ms_per_pair
     cudaFree(saved);
     if (result != LBM_OK) return result;
     if (best) *best = best_v;
-    return lbm_set_fast_variant(s, best_v);
+    return select_variant(s, best_v);
 }
 
 int lbm_get_density_distributions(lbm_solver* s, const int32_t origin[3], const int32_t size[3], void* host,

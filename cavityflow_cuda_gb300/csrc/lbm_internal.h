@@ -24,7 +24,7 @@ struct lbm_solver {
     bool macros_fresh = false;
     double* scratch = nullptr;      // reduction partials (4 per block) + result (4)
     unsigned long long* counts = nullptr;  // cavity-flag check counters [0..1], kernel error flag [2],
-                                           // step words [4] (see step_words)
+                                           // work words of the pair kernel [3], step words [4] (see step_words)
     double* host_out = nullptr;     // pinned, 4 doubles
     float* staging = nullptr;       // 16-bit storage: one packed slot cuboid
     size_t staging_elems = 0;
@@ -35,6 +35,9 @@ struct lbm_solver {
     bool fma = false;               // FP64: fused multiply-adds in the vectorised steps
     int lid_mode = 0;               // LBM_LID_INJECTION or LBM_LID_MOVING_WALL; the wall moves
                                     // while p.wall_y > 0
+    void* dd2 = nullptr;            // lbm_run's second population array (ensure_pairs)
+    bool pairs = true;              // lbm_run may take two steps a pass: no launch variant was asked for
+    bool pairs_refused = false;     // no memory for dd2
     cudaStream_t capture_stream = nullptr;
     cudaGraphExec_t graph = nullptr;
     int64_t device_bytes = 0;

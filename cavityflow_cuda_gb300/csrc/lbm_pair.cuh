@@ -1,0 +1,656 @@
+// lbm_pair.cuh -- two time steps (alpha, then beta) of the box cavity in one
+// pass over the populations.
+//
+// alpha_fast and beta_fast_* each read and write every population once, and
+// stream at 0.97 of the copy bandwidth: a pair costs two passes.  pair_step
+// reads the state once from `in` and writes the state two steps later to
+// `out`, another array of the same layout, so a pair costs one pass (two
+// pairs bring the state back to the first array).
+//
+// A block owns a tile of TX x TY cells and marches along z.  Per plane:
+//   1. a warp has TMA bring the 19 slots of the tile and of a one-cell frame
+//      around it into a shared-memory stage (one box a plane);
+//   2. the alpha threads collide tile and frame in place: population k of a
+//      cell goes to slot opp(k) of that cell, wall cells stay as they are,
+//      exactly as alpha leaves the array (the frame's cells are collided again
+//      by the neighbouring blocks: the price of not waiting for them);
+//   3. the beta threads pull what beta pulls from this plane: the five slots
+//      with c_z = +1 belong to their cells one plane below, the nine with
+//      c_z = 0 to their cells of this plane, the five with c_z = -1 to their
+//      cells one plane above.  They wait in registers until a cell has all 19;
+//      then it collides and pushes population k to slot k at x + c_k of `out`.
+// Slot k of a cell whose neighbour x - c_k is a wall is written by alpha alone
+// (nobody pushes into it): the cell copies it from the stage to `out`.  So
+// `out` gets every slot that a later step reads; slots that no step reads keep
+// what they held.  Results are bit-identical to the separate kernels.
+//
+// The three kinds of threads work on different planes at the same time, a ring
+// of stages between them: with all threads first in alpha and then in beta, a
+// block's memory and arithmetic phases took turns and a pair was no faster
+// than two separate steps (2.61 ms at 384^3 FP32 against 2.58).  A thread owns
+// two cells and collides them with paired FP32 instructions (add/mul/fma.
+// rn.f32x2: the same IEEE operation on both cells, half the instructions).
+//
+// Measured on GB300 at 384^3 (ms a pair, separate kernels -> this one): FP32
+// 2.58 -> 1.49 (76.2 GLUP/s; 93 % of the copy bandwidth for the bytes it moves,
+// 1.11x its array in and 1.0x out), BF16S 1.38 -> 1.12 and F16S 1.39 -> 1.13
+// (100 GLUP/s; issue slots and the FP32 pipe, not memory: 54 % of the former
+// are used with 20 warps a SM).
+#pragma once
+
+#include <cstdint>
+#include <type_traits>
+#include <cuda.h>
+
+#include "lbm_core.cuh"
+#include "lbm_fast.cuh"
+#include "lbm_kernels.h"
+#include "lbm_tma.cuh"
+
+namespace lbm {
+
+// ---------------------------------------------------------------------------
+// Two FP32 values in one 64-bit register pair.
+// ---------------------------------------------------------------------------
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2_make(float lo, float hi)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 f2_both(float a) { return f2_make(a, a); }
+__device__ __forceinline__ void f2_split(F2 a, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b)
+{
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// Product with a constant, as two scalar multiplies: given a constant operand,
+// ptxas contracts mul.rn.f32x2 and the add or sub that follows into one fused
+// multiply-add (the scalar mul.rn.f32 it leaves alone, and so it does products
+// of two variables), which changes the result.  The FP32 pipe takes as long for
+// two scalar operations as for a paired one.
+__device__ __forceinline__ F2 f2_scale(float c, F2 a)
+{
+    float lo, hi;
+    f2_split(a, lo, hi);
+    return f2_make(__fmul_rn(c, lo), __fmul_rn(c, hi));
+}
+
+// relax_pair (lbm_core.cuh) on two cells: the same operations in the same
+// order, except that P + (-3 s) is written P - 3 s, which is the same value.
+__device__ __forceinline__ void relax_pair2(F2& fp, F2& fm, float w, F2 P, F2 s, float inv_tau)
+{
+    const F2 s2 = s * s;
+    const F2 t = f2_scale(4.5f, s2);
+    const F2 a = f2_scale(3.0f, s);
+    const F2 ep = f2_scale(w, (P + a) + t);
+    const F2 em = f2_scale(w, (P - a) + t);
+    fp = fp + f2_scale(inv_tau, ep - fp);
+    fm = fm + f2_scale(inv_tau, em - fm);
+}
+
+// collide_fluid<float> on two cells.
+__device__ __forceinline__ void collide_fluid2(F2* f, float inv_tau)
+{
+    F2 r = f[0], x = f[0], y, z;
+    r = r + f[1];  x = x - f[1];
+    r = r + f[2];  y = f[2];
+    r = r + f[3];  y = y - f[3];
+    r = r + f[4];  x = x + f[4];  y = y + f[4];
+    r = r + f[5];  x = x - f[5];  y = y - f[5];
+    r = r + f[6];  x = x + f[6];  y = y - f[6];
+    r = r + f[7];  x = x - f[7];  y = y + f[7];
+    r = r + f[8];  x = x + f[8];  z = f[8];
+    r = r + f[9];  x = x - f[9];  z = z - f[9];
+    r = r + f[10]; x = x + f[10]; z = z - f[10];
+    r = r + f[11]; x = x - f[11]; z = z + f[11];
+    r = r + f[12]; y = y + f[12]; z = z + f[12];
+    r = r + f[13]; y = y - f[13]; z = z - f[13];
+    r = r + f[14]; y = y + f[14]; z = z - f[14];
+    r = r + f[15]; y = y - f[15]; z = z + f[15];
+    r = r + f[16]; z = z + f[16];
+    r = r + f[17]; z = z - f[17];
+    r = r + f[18];
+    const F2 vel2 = x * x + y * y + z * z;
+    const F2 P = r - f2_scale(1.5f, vel2);
+    constexpr float wa = 1.0f / 18.0f, wd = 1.0f / 36.0f;
+    relax_pair2(f[0], f[1], wa, P, x, inv_tau);
+    relax_pair2(f[2], f[3], wa, P, y, inv_tau);
+    relax_pair2(f[4], f[5], wd, P, x + y, inv_tau);
+    relax_pair2(f[6], f[7], wd, P, x - y, inv_tau);
+    relax_pair2(f[8], f[9], wd, P, x + z, inv_tau);
+    relax_pair2(f[10], f[11], wd, P, x - z, inv_tau);
+    relax_pair2(f[12], f[13], wd, P, y + z, inv_tau);
+    relax_pair2(f[14], f[15], wd, P, y - z, inv_tau);
+    relax_pair2(f[16], f[17], wa, P, z, inv_tau);
+    f[18] = f[18] + f2_scale(inv_tau, f2_scale(1.0f / 3.0f, P) - f[18]);
+}
+
+// relax_pair_shifted / collide_shifted on two cells.
+__device__ __forceinline__ void relax_pair_shifted2(F2& sp, F2& sm, float w3, float w45, F2 wP, F2 u, F2 omega)
+{
+    const F2 even = f2_fma(f2_both(w45), u * u, wP);
+    const F2 odd = f2_scale(w3, u);
+    sp = f2_fma(omega, (even + odd) - sp, sp);
+    sm = f2_fma(omega, (even - odd) - sm, sm);
+}
+
+template <int E>
+__device__ __forceinline__ void collide_shifted2(F2* s, F2 omega)
+{
+    const F2 a01 = s[0] + s[1], d01 = s[0] - s[1];
+    const F2 a23 = s[2] + s[3], d23 = s[2] - s[3];
+    const F2 a45 = s[4] + s[5], d45 = s[4] - s[5];
+    const F2 a67 = s[6] + s[7], d67 = s[6] - s[7];
+    const F2 a89 = s[8] + s[9], d89 = s[8] - s[9];
+    const F2 a1011 = s[10] + s[11], d1011 = s[10] - s[11];
+    const F2 a1213 = s[12] + s[13], d1213 = s[12] - s[13];
+    const F2 a1415 = s[14] + s[15], d1415 = s[14] - s[15];
+    const F2 a1617 = s[16] + s[17], d1617 = s[16] - s[17];
+    const F2 drho = ((a01 + a23) + (a45 + a67)) + ((a89 + a1011) + (a1213 + a1415)) + (a1617 + s[18]);
+    const F2 jx = ((d01 + d45) + (d67 + d89)) + d1011;
+    const F2 jy = ((d23 + d45) - d67) + (d1213 + d1415);
+    const F2 jz = ((d89 - d1011) + (d1213 - d1415)) + d1617;
+    const F2 vel2 = f2_fma(jz, jz, f2_fma(jy, jy, jx * jx));
+    constexpr float inv_scale = 1.0f / (float)(1u << E);
+    const F2 P = f2_fma(f2_both(-1.5f * inv_scale), vel2, drho);
+    constexpr float wa = 1.0f / 18.0f, wd = 1.0f / 36.0f;
+    const F2 waP = f2_scale(wa, P), wdP = f2_scale(wd, P);
+    constexpr float wa3 = 3.0f * wa, wa45 = (4.5f * wa) * inv_scale, wd3 = 3.0f * wd, wd45 = (4.5f * wd) * inv_scale;
+    relax_pair_shifted2(s[0], s[1], wa3, wa45, waP, jx, omega);
+    relax_pair_shifted2(s[2], s[3], wa3, wa45, waP, jy, omega);
+    relax_pair_shifted2(s[4], s[5], wd3, wd45, wdP, jx + jy, omega);
+    relax_pair_shifted2(s[6], s[7], wd3, wd45, wdP, jx - jy, omega);
+    relax_pair_shifted2(s[8], s[9], wd3, wd45, wdP, jx + jz, omega);
+    relax_pair_shifted2(s[10], s[11], wd3, wd45, wdP, jx - jz, omega);
+    relax_pair_shifted2(s[12], s[13], wd3, wd45, wdP, jy + jz, omega);
+    relax_pair_shifted2(s[14], s[15], wd3, wd45, wdP, jy - jz, omega);
+    relax_pair_shifted2(s[16], s[17], wa3, wa45, waP, jz, omega);
+    s[18] = f2_fma(omega, f2_scale(1.0f / 3.0f, P) - s[18], s[18]);
+}
+
+// One step's cell rule on two cells of a row: wall correction, then the lid's
+// equilibrium or the collision.
+template <class St>
+__device__ __forceinline__ void cell_rule2(F2* f, bool lid, bool wall, float inv_tau, float lid_u)
+{
+    if (wall) {
+        const F2 du = f2_both(wall_shift<St>(lid_u));
+        f[5] = f[5] - du;
+        f[6] = f[6] + du;
+    }
+    if (lid) {
+        float e[Q];
+        inject_step<St>(e, St::shifted ? 0.0f : 1.0f, lid_u);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) f[k] = f2_both(e[k]);
+    } else if constexpr (St::shifted) {
+        collide_shifted2<St::kStepLog2>(f, f2_both(inv_tau));
+    } else {
+        collide_fluid2(f, inv_tau);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Two neighbouring stored populations of a slot: 8 bytes (FP32) or one word.
+// ---------------------------------------------------------------------------
+template <class St, bool kWide = sizeof(typename St::bits) == 4>
+struct Two;
+
+template <class St>
+struct Two<St, true> {
+    using raw = unsigned long long;
+    __device__ static raw load(const float* p) { return *reinterpret_cast<const raw*>(p); }
+    __device__ static void store(float* p, raw r) { *reinterpret_cast<raw*>(p) = r; }
+    __device__ static raw join(float a, float b) { return f2_make(a, b).v; }
+    __device__ static float first(raw r)
+    {
+        float a, b;
+        f2_split(F2{r}, a, b);
+        return a;
+    }
+    __device__ static float second(raw r)
+    {
+        float a, b;
+        f2_split(F2{r}, a, b);
+        return b;
+    }
+    // the cells at p[DX] and p[DX + SEP]
+    template <int DX, int SEP>
+    __device__ static raw load_at(const float* p)
+    {
+        return join(p[DX], p[DX + SEP]);
+    }
+    __device__ static F2 widen(raw r) { return F2{r}; }
+    __device__ static raw narrow(F2 v, uint32_t, uint32_t, int) { return v.v; }
+};
+
+template <class St>
+struct Two<St, false> {
+    using raw = uint32_t;
+    using bits = unsigned short;
+    __device__ static raw load(const bits* p) { return *reinterpret_cast<const raw*>(p); }
+    __device__ static void store(bits* p, raw r) { *reinterpret_cast<raw*>(p) = r; }
+    __device__ static raw join(bits a, bits b) { return (raw)a | ((raw)b << 16); }
+    __device__ static bits first(raw r) { return (bits)(r & 0xffffu); }
+    __device__ static bits second(raw r) { return (bits)(r >> 16); }
+    // the cells at p[DX] and p[DX + 1], p aligned to a word (SEP is 1)
+    template <int DX, int SEP>
+    __device__ static raw load_at(const bits* p)
+    {
+        if constexpr (DX == 0) return load(p);
+        else if constexpr (DX == 1) return __byte_perm(load(p), load(p + 2), 0x5432);
+        else return __byte_perm(load(p - 2), load(p), 0x5432);
+    }
+    __device__ static F2 widen(raw r) { return f2_make(St::load_step(first(r)), St::load_step(second(r))); }
+    __device__ static raw narrow(F2 v, uint32_t h0, uint32_t h1, int k)
+    {
+        float a, b;
+        f2_split(v, a, b);
+        return pk_two<St>(pk_pre<St>(a, h0, k), pk_pre<St>(b, h1, k));
+    }
+};
+
+// Geometry of one shape: TX x TY cells, NST stages.  A stage is a box of the
+// population array: all 19 slots, the tile's rows and one on either side, and
+// from 16 bytes left of the tile's first cell to 16 bytes right of its last
+// (TMA copies start and end on 16-byte boundaries).
+template <class St, int TX, int TY, int NST>
+struct PairShape {
+    using bits = typename St::bits;
+    static constexpr int LX = 16 / (int)sizeof(bits);            // column of the tile's first cell
+    static constexpr int W = TX + 2 * LX;                        // stage row
+    static constexpr int SLOT = (TY + 2) * W;                    // stage slot
+    static constexpr int STAGE = (Q * SLOT * (int)sizeof(bits) + 127) / 128 * 128 / (int)sizeof(bits);
+    static constexpr uint32_t BYTES = (uint32_t)(Q * SLOT * sizeof(bits));
+    static constexpr int PAIRS = (TY + 2) * (TX / 2);              // pairs of cells of tile rows -1 .. TY
+    static constexpr int NA = (PAIRS + 2 * (TY + 2) + 31) / 32 * 32;  // alpha threads: also the frame's columns
+    static constexpr int NB = TY * (TX / 2);                       // beta threads
+    static constexpr int THREADS = NA + NB + 32;                 // and the warp that issues the copies
+    static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(bits) + NST * (sizeof(uint64_t) + sizeof(int));
+    // the two cells of a beta thread: FP32 half a row apart, so that each access
+    // of a warp is one run of 4-byte elements whatever the shift; 16-bit neighbours,
+    // one word
+    static constexpr int SEP = sizeof(bits) == 4 ? TX / 2 : 1;
+    static_assert(NB % 32 == 0, "whole warps");
+    static_assert(2 * NST <= 15, "named barriers");
+};
+
+// Named barriers, as a producer and a consumer use them: `arrive` does not wait.
+__device__ __forceinline__ void named_sync(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// The work of one launch: the tiles of every z chunk, chunks slowest.  Blocks
+// are persistent and take the next item from a counter, so that at any time
+// they work on neighbouring tiles of the same planes and find each other's
+// frames in L2; a block's copies run ahead into its next item.
+struct PairWork {
+    int tiles_x, tiles, items;  // tiles of a row, of a plane; items in all
+    int zc;                     // planes of a chunk
+    int* next;                  // [0] items taken beyond the first of each block, [1] blocks done; zero between launches
+};
+struct PairItem {
+    int x0, y0, za, zb;  // first cell, first and last plane
+};
+template <int TX, int TY>
+__device__ __forceinline__ PairItem pair_item(const PairWork& w, const Grid& g, int item)
+{
+    const int chunk = item / w.tiles, t = item - chunk * w.tiles;
+    const int ty = t / w.tiles_x, tx = t - ty * w.tiles_x;
+    const int za = 1 + chunk * w.zc;
+    return {1 + tx * TX, 1 + ty * TY, za, min(g.nz, za + w.zc - 1)};
+}
+// Waits until the phase with `parity` of `bar` has completed, at most limit_ns
+// (tma::mbar_wait with the hardware's own wait between the looks).
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns)
+{
+    uint64_t deadline = 0;
+    for (;;) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(tma::smem_addr(bar)), "r"(parity), "r"(100000u)  // ns the hardware may suspend the thread
+            : "memory");
+        if (done) return true;
+        const uint64_t now = tma::now_ns();
+        if (deadline == 0) deadline = now + limit_ns;
+        else if (now > deadline) return false;
+    }
+}
+
+// Where the slots of `out` are: own[k] + o is slot k of the cell at byte o of
+// its slot, push[k] + o the place in slot k, one plane below, that the cell
+// pushes population k to.  Uniform bases and a 32-bit offset a thread: one
+// address per access instead of a 64-bit sum.
+struct PairSlots {
+    char* own[Q];
+    char* push[Q];
+};
+inline PairSlots pair_slots(void* out, const Grid& g, int elem)
+{
+    PairSlots s;
+    for (int k = 0; k < Q; ++k) {
+        s.own[k] = static_cast<char*>(out) + (long long)k * g.S * elem;
+        s.push[k] = s.own[k] + ((dir_z(k) - 1) * g.PY + dir_y(k) * g.P + dir_x(k)) * elem;
+    }
+    return s;
+}
+
+// The slots that point away from the low (SIGN 1) or high (-1) wall of an axis.
+template <int AXIS, int SIGN>
+struct FromFace {
+    __host__ __device__ static constexpr bool at(int k) { return (AXIS == 0 ? dir_x(k) : AXIS == 1 ? dir_y(k) : dir_z(k)) == SIGN; }
+};
+
+// Index of slot k among the slots of its c_z.
+__host__ __device__ constexpr int z_rank(int k)
+{
+    int n = 0;
+    for (int q = 0; q < k; ++q) n += dir_z(q) == dir_z(k);
+    return n;
+}
+
+// The copying warp: takes items and brings the planes za - 1 .. zb + 1 of each
+// into the stages, as beta gives them back.  item_of[s] tells the others what
+// stage s holds; -1 ends the block.
+template <class St, int TX, int TY, int NST>
+__device__ __forceinline__ void pair_copy(const CUtensorMap* map, const Grid& g, const PairWork& w,
+                                          typename St::bits* smem, uint64_t* full, int* item_of)
+{
+    using S = PairShape<St, TX, TY, NST>;
+    const bool lead = (threadIdx.x & 31) == 0;
+    int stage = 0, used = 0, item = (int)blockIdx.x;
+#pragma unroll 1
+    while (item < w.items) {
+        const PairItem it = pair_item<TX, TY>(w, g, item);
+        int next = 0;
+#pragma unroll 1
+        for (int p = it.za - 1; p <= it.zb + 1; ++p) {
+            if (lead && p == it.zb) next = atomicAdd(&w.next[0], 1);
+            if (used == NST) named_sync(1 + NST + stage, S::NB + 32);
+            else ++used;
+            if (lead) {
+                item_of[stage] = item;
+                tma::fence_proxy_async();  // alpha's and beta's accesses to the stage, before the copy overwrites it
+                tma::mbar_arrive_expect_tx(&full[stage], S::BYTES);
+                asm volatile(
+                    "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
+                    "%5}], [%6];" ::"r"(tma::smem_addr(smem + stage * S::STAGE)),
+                    "l"(map), "r"(g.xoff + it.x0 - S::LX), "r"(it.y0 - 1), "r"(p), "r"(0),
+                    "r"(tma::smem_addr(&full[stage]))
+                    : "memory");
+            }
+            stage = stage + 1 == NST ? 0 : stage + 1;
+        }
+        item = __shfl_sync(0xffffffffu, next, 0) + (int)gridDim.x;
+    }
+    if (used == NST) named_sync(1 + NST + stage, S::NB + 32);
+    else ++used;
+    if (lead) {
+        item_of[stage] = -1;
+        tma::mbar_arrive(&full[stage]);
+        if (atomicAdd(&w.next[1], 1) == (int)gridDim.x - 1) {  // every block has taken its last item
+            w.next[0] = 0;
+            w.next[1] = 0;
+        }
+    }
+    for (int s = 0; s < used; ++s) {  // beta gives back every stage, the last ones to nobody but this warp
+        stage = stage + 1 >= used ? 0 : stage + 1;
+        named_sync(1 + NST + stage, S::NB + 32);
+    }
+}
+
+// Alpha threads: collide the cells of a stage in place.
+template <class St, int TX, int TY, int NST>
+__device__ __forceinline__ void pair_alpha(const Grid& g, const float inv_tau, const float lid_u, const int lid_y,
+                                           const int wall_y, const PairWork& w, const uint32_t step,
+                                           typename St::bits* __restrict__ smem, uint64_t* full,
+                                           const int* item_of, int* __restrict__ err)
+{
+    using S = PairShape<St, TX, TY, NST>;
+    using bits = typename St::bits;
+    using two = Two<St>;
+    // Pairs of tile rows -1 .. TY, then two cells left and two right of each of
+    // these rows, of which the frame has the nearer one; the other cell of such
+    // a pair is collided from whatever the stage holds, and nothing reads it.
+    const int tid = (int)threadIdx.x;
+    const bool column = tid >= S::PAIRS;
+    const int c = tid - S::PAIRS;
+    const int ry = column ? (c < TY + 2 ? c : c - (TY + 2)) : tid / (TX / 2);
+    const int px = !column ? tid % (TX / 2) : c < TY + 2 ? -1 : TX / 2;
+    bits* const own = smem + ry * S::W + S::LX + 2 * px;
+    int stage = 0;
+    uint32_t phase = 0;
+    uint64_t limit_ns = tma::kWaitLimitNs;
+    int item = -1, p = 0, y = 0, xa = 0;
+    bool work = false, both = false, lid = false, wall = false;
+#pragma unroll 1
+    for (;;) {
+        if (!pair_wait(&full[stage], phase, limit_ns)) {  // reported; the block runs on to its end
+            atomicOr(err, 4);
+            limit_ns = 1000000;
+        }
+        const int now = *(const volatile int*)&item_of[stage];
+        ++p;
+        if (now != item) {  // another tile's first plane
+            if (now < 0) break;
+            item = now;
+            const PairItem it = pair_item<TX, TY>(w, g, item);
+            p = it.za - 1;
+            y = it.y0 - 1 + ry;
+            xa = it.x0 + 2 * px;
+            const int x = column && px < 0 ? xa + 1 : xa;  // the cell that decides
+            work = ry <= TY + 1 && y >= 1 && y <= g.ny && x >= 1 && x <= g.nx;
+            both = column || xa < g.nx;
+            lid = y == lid_y;
+            wall = y == wall_y;
+        }
+        bits* const sb = own + stage * S::STAGE;
+        if (p >= 1 && p <= g.nz && work) {
+            uint32_t ha = 0, hb = 0;
+            if constexpr (St::stochastic) {
+                const uint32_t rh = sr_hash((uint32_t)g.ref(0, y, p), step);
+                ha = sr_cell(rh, xa);
+                hb = sr_cell(rh, xa + 1);
+            }
+            F2 f[Q];
+#pragma unroll
+            for (int k = 0; k < Q; ++k) f[k] = two::widen(two::load(sb + k * S::SLOT));
+            cell_rule2<St>(f, lid, wall, inv_tau, lid_u);
+            if (both) {
+#pragma unroll
+                for (int k = 0; k < Q; ++k) two::store(sb + opp(k) * S::SLOT, two::narrow(f[k], ha, hb, k));
+            } else {  // the second cell is the wall behind the row's end
+#pragma unroll
+                for (int k = 0; k < Q; ++k) sb[opp(k) * S::SLOT] = two::first(two::narrow(f[k], ha, hb, k));
+            }
+        }
+        named_arrive(1 + stage, S::NA + S::NB);
+        if (++stage == NST) {
+            stage = 0;
+            phase ^= 1;
+        }
+    }
+    named_arrive(1 + stage, S::NA + S::NB);
+}
+
+// Beta threads: pull, collide, push to `out`.
+template <class St, int TX, int TY, int NST>
+__device__ __forceinline__ void pair_beta(const PairSlots& slots, const Grid& g, const float inv_tau,
+                                          const float lid_u, const int lid_y, const int wall_y, const PairWork& w,
+                                          const uint32_t step, typename St::bits* __restrict__ smem, const int* item_of)
+{
+    using S = PairShape<St, TX, TY, NST>;
+    using bits = typename St::bits;
+    using two = Two<St>;
+    using raw = typename two::raw;
+    const int tid = (int)threadIdx.x - S::NA;
+    const int ry = tid / (TX / 2), px = tid % (TX / 2);
+    constexpr int SEP = S::SEP;
+    const int dx = SEP == 1 ? 2 * px : px;
+    const bits* const own = smem + (ry + 1) * S::W + S::LX + dx;
+    const uint32_t pitch = (uint32_t)(g.PY * (long long)sizeof(bits));
+    raw c0[9], m1[5], m2[5];
+    int stage = 0, item = -1, p = 0, za = 0, zb = 0, y = 0, xa = 0;
+    bool tile = false, vb = false, lid = false, wall = false, edge = false;
+    uint32_t off = 0;  // of (xa, y, p) in a slot, bytes
+#pragma unroll 1
+    for (;;) {
+        named_sync(1 + stage, S::NA + S::NB);
+        const int now = *(const volatile int*)&item_of[stage];
+        ++p;
+        off += pitch;
+        if (now != item) {  // another tile's first plane
+            if (now < 0) break;
+            item = now;
+            const PairItem it = pair_item<TX, TY>(w, g, item);
+            za = it.za;
+            zb = it.zb;
+            p = za - 1;
+            y = it.y0 + ry;
+            xa = it.x0 + dx;
+            tile = y <= g.ny && xa <= g.nx;
+            vb = xa + SEP <= g.nx;
+            lid = y == lid_y;
+            wall = y == wall_y;
+            edge = xa == 1 || xa == g.nx || xa + SEP == g.nx || y == 1 || y == g.ny;
+            off = (uint32_t)(g.idx(xa, y, p) * (long long)sizeof(bits));
+        }
+        if (tile) {
+            const bits* const sb = own + stage * S::STAGE;
+            if (p > za) {  // the cells of plane p - 1 have all their populations now
+                F2 f[Q];
+                static_for<0, Q>([&](auto kc) {
+                    constexpr int k = decltype(kc)::value;
+                    raw r;
+                    if constexpr (dir_z(k) == 1) r = two::template load_at<dir_x(k), SEP>(sb + k * S::SLOT + dir_y(k) * S::W);
+                    else if constexpr (dir_z(k) == 0) r = c0[z_rank(k)];
+                    else r = m1[z_rank(k)];
+                    f[opp(k)] = two::widen(r);
+                });
+                cell_rule2<St>(f, lid, wall, inv_tau, lid_u);
+                uint32_t ha = 0, hb = 0;
+                if constexpr (St::stochastic) {
+                    const uint32_t rh = sr_hash((uint32_t)g.ref(0, y, p - 1), step + 1);
+                    ha = sr_cell(rh, xa);
+                    hb = sr_cell(rh, xa + SEP);
+                }
+                if (vb) {
+                    static_for<0, Q>([&](auto kc) {
+                        constexpr int k = decltype(kc)::value;
+                        const raw r = two::narrow(f[k], ha, hb, k);
+                        bits* const q = reinterpret_cast<bits*>(slots.push[k] + off);
+                        if constexpr (SEP == 1 && dir_x(k) == 0) {
+                            __stcs(reinterpret_cast<raw*>(q), r);
+                        } else {
+                            __stcs(q, two::first(r));
+                            __stcs(q + SEP, two::second(r));
+                        }
+                    });
+                } else {
+                    static_for<0, Q>([&](auto kc) {
+                        constexpr int k = decltype(kc)::value;
+                        *reinterpret_cast<bits*>(slots.push[k] + off) = two::first(two::narrow(f[k], ha, hb, k));
+                    });
+                }
+            }
+            // what beta pulls from this plane for the cells of this plane and of the next
+            static_for<0, Q>([&](auto kc) {
+                constexpr int k = decltype(kc)::value;
+                if constexpr (dir_z(k) == 0) {
+                    c0[z_rank(k)] = two::template load_at<dir_x(k), SEP>(sb + k * S::SLOT + dir_y(k) * S::W);
+                }
+                if constexpr (dir_z(k) == -1) {
+                    m1[z_rank(k)] = m2[z_rank(k)];
+                    m2[z_rank(k)] = two::template load_at<dir_x(k), SEP>(sb + k * S::SLOT + dir_y(k) * S::W);
+                }
+            });
+            // slots that only alpha writes: the neighbour they would come from is a wall
+            if (p >= za && p <= zb && (edge || p == 1 || p == g.nz)) {
+                auto keep = [&](auto want, bool first, bool second) {
+                    static_for<0, Q>([&](auto kc) {
+                        constexpr int k = decltype(kc)::value;
+                        if constexpr (decltype(want)::at(k)) {
+                            bits* const q = reinterpret_cast<bits*>(slots.own[k] + off);
+                            if (first) q[0] = sb[k * S::SLOT];
+                            if (second) q[SEP] = sb[k * S::SLOT + SEP];
+                        }
+                    });
+                };
+                if (xa == 1) keep(FromFace<0, 1>{}, true, false);
+                if (xa == g.nx || xa + SEP == g.nx) keep(FromFace<0, -1>{}, xa == g.nx, xa + SEP == g.nx);
+                if (y == 1) keep(FromFace<1, 1>{}, true, vb);
+                if (y == g.ny) keep(FromFace<1, -1>{}, true, vb);
+                if (p == 1) keep(FromFace<2, 1>{}, true, vb);
+                if (p == g.nz) keep(FromFace<2, -1>{}, true, vb);
+            }
+        }
+        named_arrive(1 + NST + stage, S::NB + 32);
+        stage = stage + 1 == NST ? 0 : stage + 1;
+    }
+    named_arrive(1 + NST + stage, S::NB + 32);
+}
+
+template <class St, int TX, int TY, int NST>
+__global__ void __launch_bounds__(PairShape<St, TX, TY, NST>::THREADS, 1)
+    pair_step(const __grid_constant__ CUtensorMap map, const __grid_constant__ PairSlots slots, const Grid g,
+              const float inv_tau, const float lid_u, const int lid_y, const int wall_y,
+              const uint32_t* __restrict__ step_base, const uint32_t step_off, const PairWork w,
+              int* __restrict__ err)
+{
+    using S = PairShape<St, TX, TY, NST>;
+    extern __shared__ __align__(128) unsigned char pair_smem[];
+    auto* const smem = reinterpret_cast<typename St::bits*>(pair_smem);
+    uint64_t* const full = reinterpret_cast<uint64_t*>(smem + NST * S::STAGE);
+    int* const item_of = reinterpret_cast<int*>(full + NST);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NST; ++s) tma::mbar_init(&full[s], 1);
+        tma::fence_mbar_init();
+    }
+    __syncthreads();
+    const uint32_t step = step_of<St>(step_base, step_off);
+    if (threadIdx.x < S::NA)
+        pair_alpha<St, TX, TY, NST>(g, inv_tau, lid_u, lid_y, wall_y, w, step, smem, full, item_of, err);
+    else if (threadIdx.x < S::NA + S::NB)
+        pair_beta<St, TX, TY, NST>(slots, g, inv_tau, lid_u, lid_y, wall_y, w, step, smem, item_of);
+    else
+        pair_copy<St, TX, TY, NST>(&map, g, w, smem, full, item_of);
+}
+
+}  // namespace lbm
