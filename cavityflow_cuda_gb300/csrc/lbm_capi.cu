@@ -83,8 +83,9 @@ constexpr int kGraphPairs = 32;  // alpha/beta pairs per captured graph
 // vectors in both kernels and beta's shifted windows accessed directly (no
 // exchange), FP16 (both roundings) with a 16-byte alpha and an 8-byte direct
 // beta, BF16 with 16-byte vectors and the block-wide beta exchange.  FP64 is
-// bound by FP64 arithmetic, where the shapes tie; it keeps 8-byte vectors
-// (one cell).
+// bound by FP64 arithmetic: one cell a thread (8 bytes), two-warp blocks and
+// direct windows (2.06 ms a pair at 160^3; variant 3, the warp exchange in
+// eight-warp blocks, 2.14).
 }  // namespace
 
 // Batch and server rows are packed for 8-byte vectors (kPackedX1Align), so
@@ -92,11 +93,10 @@ constexpr int kGraphPairs = 32;  // alpha/beta pairs per captured graph
 // seeded 512-cavity workload the direct beta windows in two-warp blocks
 // (variant 13) are fastest for FP32, the packed 16-bit beta at <= 128
 // registers (22: the batch kernel's own state spills the 102-register
-// shape) for the 16-bit storages, the FP64 warp exchange (3) for FP64.
+// shape) for the 16-bit storages.
 int lbm_detail::default_batch_variant(int storage)
 {
     switch (storage) {
-    case LBM_STORAGE_F64: return 3;
     case LBM_STORAGE_F16S:
     case LBM_STORAGE_BF16S:
     case LBM_STORAGE_F16SR: return 22;
@@ -111,7 +111,7 @@ int lbm_detail::default_variant(int storage)
     case LBM_STORAGE_F16S: return 20;
     case LBM_STORAGE_BF16S: return 20;
     case LBM_STORAGE_F16SR: return 20;
-    default: return 3;
+    default: return 13;
     }
 }
 

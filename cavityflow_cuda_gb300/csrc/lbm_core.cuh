@@ -9,9 +9,12 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+
+#include "lbm_f64.cuh"
 
 namespace lbm {
 
@@ -488,12 +491,63 @@ __device__ __forceinline__ void collide_shifted(float* s, float omega)
     s[18] = __fmaf_rn(omega, (1.0f / 3.0f) * P - s[18], s[18]);
 }
 
+// ---------------------------------------------------------------------------
+// collide_fluid<double> with its multiplications on the integer units
+// (lbm_f64.cuh): the same operations in the same order, so the same bits.
+// ---------------------------------------------------------------------------
+
+// f + inv_tau * (e - f); inv_tau positive and exp_ok.
+__device__ __forceinline__ double relax_f64(double f, double e, double inv_tau)
+{
+    const double d = e - f;
+    if (f64::is_zero(d)) return f + d;
+    return f + (f64::exp_ok(d) ? f64::mul(inv_tau, d) : inv_tau * d);
+}
+
+// relax_pair; s and inv_tau exp_ok.  P + (-3 s) is P - 3 s.
+__device__ __forceinline__ void relax_pair_f64(double& fp, double& fm, double w, double P, double s, double inv_tau)
+{
+    const double t = f64::mul4_5(f64::mul(s, s));
+    const double a = f64::mul3(s);
+    const double p = (P + a) + t, m = (P - a) + t;
+    const bool ok = f64::exp_ok(p) && f64::exp_ok(m);
+    fp = relax_f64(fp, ok ? f64::mul(w, p) : w * p, inv_tau);
+    fm = relax_f64(fm, ok ? f64::mul(w, m) : w * m, inv_tau);
+}
+
+__device__ __forceinline__ void collide_fluid_f64(double* f, double inv_tau)
+{
+    double rho, vx, vy, vz;
+    moments(f, rho, vx, vy, vz);
+    const double xpy = vx + vy, xmy = vx - vy, xpz = vx + vz, xmz = vx - vz, ypz = vy + vz, ymz = vy - vz;
+    const bool ok = f64::exp_ok(vx) && f64::exp_ok(vy) && f64::exp_ok(vz) && f64::exp_ok(xpy) && f64::exp_ok(xmy) &&
+                    f64::exp_ok(xpz) && f64::exp_ok(xmz) && f64::exp_ok(ypz) && f64::exp_ok(ymz) && f64::exp_ok(inv_tau);
+    if (!ok) {
+        collide_fluid(f, inv_tau);
+        return;
+    }
+    const double vel2 = f64::mul(vx, vx) + f64::mul(vy, vy) + f64::mul(vz, vz);
+    const double P = rho - f64::mul1_5(vel2);
+    const double wa = 1.0 / 18.0, wd = 1.0 / 36.0;
+    relax_pair_f64(f[0], f[1], wa, P, vx, inv_tau);
+    relax_pair_f64(f[2], f[3], wa, P, vy, inv_tau);
+    relax_pair_f64(f[4], f[5], wd, P, xpy, inv_tau);
+    relax_pair_f64(f[6], f[7], wd, P, xmy, inv_tau);
+    relax_pair_f64(f[8], f[9], wd, P, xpz, inv_tau);
+    relax_pair_f64(f[10], f[11], wd, P, xmz, inv_tau);
+    relax_pair_f64(f[12], f[13], wd, P, ypz, inv_tau);
+    relax_pair_f64(f[14], f[15], wd, P, ymz, inv_tau);
+    relax_pair_f64(f[16], f[17], wa, P, vz, inv_tau);
+    f[18] = relax_f64(f[18], f64::exp_ok(P) ? f64::mul(1.0 / 3.0, P) : (1.0 / 3.0) * P, inv_tau);
+}
+
 // Collision dispatch by storage: the reference's arithmetic for F64/F32, the
 // fused form above for the shifted 16-bit modes.
 template <class St>
 __device__ __forceinline__ void collide(typename St::T* f, typename St::T inv_tau)
 {
     if constexpr (St::shifted) collide_shifted<St::kStepLog2>(f, inv_tau);
+    else if constexpr (std::is_same<St, F64>::value) collide_fluid_f64(f, inv_tau);
     else collide_fluid(f, inv_tau);
 }
 
