@@ -122,8 +122,8 @@ inline int storage_elem_bytes(int storage)
 cudaError_t launch_fast_step(int storage, int variant, bool alpha, void* dd, const Grid& g, const Params& p,
                              int lid_y, int* err, cudaStream_t st);
 // Two steps, alpha then beta, in one pass from the populations `in` to `out`, an
-// array of the same layout (lbm_pair.cuh).  F32 (unfused), F16S and
-// BF16S.  `work` is two device words that are zero between launches.
+// array of the same layout (lbm_pair.cuh).  F32 (unfused) and the
+// 16-bit storages.  `work` is two device words that are zero between launches.
 cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid& g, const Params& p, int lid_y,
                              int* work, int* err, cudaStream_t st);
 // Whether that kernel can run on this domain and takes less time than the

@@ -9,17 +9,19 @@ namespace lbm {
 
 namespace {
 
-// One shape for all storages: 64 x 8 cells (a warp's pairs are one row; two
-// beta warps and about three alpha warps on each of the SM's four schedulers
-// at 96 registers).  32 x 8 and 32 x 4 tiles in one to three blocks a SM
-// collide more frame cells and ran 15-30 % slower, 64 x 16 does not fit the
-// registers.  Stages: as many as shared memory holds, up to six.
-constexpr int kTX = 64, kTY = 8;
+// Tiles of 64 cells (a warp's pairs are one row) by 8 rows for FP32 (20 warps
+// at 96 registers) and by 10 for the 16-bit storages (24 warps at 80: more
+// warps and fewer frame rows; F16SR 87.4 GLUP/s at 384^3 against 83.6 with 8
+// rows, where FP32 spills and falls from 76 to 68).  32 x 8 and 32 x 4 tiles in
+// one to three blocks a SM collide more frame cells and ran 15-30 % slower.
+// Stages: as many as shared memory holds, up to five.
+constexpr int kTX = 64;
 template <class St>
-constexpr int stages()
-{
-    return sizeof(typename St::bits) == 4 ? 4 : 6;
-}
+struct Shape {
+    static constexpr int TY = sizeof(typename St::bits) == 4 ? 8 : 10;
+    static constexpr int NST = sizeof(typename St::bits) == 4 ? 4 : 5;
+};
+int tile_rows(int elem) { return elem == 4 ? Shape<F32>::TY : Shape<F16S>::TY; }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 {
@@ -56,11 +58,12 @@ struct Split {
     int zc;
     long long planes;  // of the busiest block
 };
-Split split(const Grid& g, int sms)
+Split split(const Grid& g, int elem, int sms)
 {
+    const int rows = tile_rows(elem);
     Split s;
     s.tiles_x = (g.nx + kTX - 1) / kTX;
-    s.tiles = s.tiles_x * ((g.ny + kTY - 1) / kTY);
+    s.tiles = s.tiles_x * ((g.ny + rows - 1) / rows);
     double best = 0;
     for (int zc = 32; zc >= 8; --zc) {
         const long long chunks = (g.nz + zc - 1) / zc;
@@ -81,25 +84,25 @@ cudaError_t launch(const void* in, void* out, const Grid& g, const Params& p, in
                    cudaStream_t st)
 {
     using bits = typename St::bits;
-    constexpr int NST = stages<St>();
-    using S = PairShape<St, kTX, kTY, NST>;
+    constexpr int TY = Shape<St>::TY, NST = Shape<St>::NST;
+    using S = PairShape<St, kTX, TY, NST>;
     const auto encode = encode_fn();
     const int sms = sm_count();
     if (!encode || sms < 1) return cudaErrorNotSupported;
     constexpr cuuint64_t eb = sizeof(bits);
     const cuuint64_t dims[4] = {(cuuint64_t)g.P, (cuuint64_t)g.ny + 2, (cuuint64_t)g.nz + 2, (cuuint64_t)Q};
     const cuuint64_t strides[3] = {(cuuint64_t)g.P * eb, (cuuint64_t)g.PY * eb, (cuuint64_t)g.S * eb};
-    const cuuint32_t box[4] = {(cuuint32_t)S::W, kTY + 2, 1, (cuuint32_t)Q}, unit[4] = {1, 1, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)S::W, TY + 2, 1, (cuuint32_t)Q}, unit[4] = {1, 1, 1, 1};
     CUtensorMap map;
     if (encode(&map, eb == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 4,
                const_cast<void*>(in), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    auto kern = pair_step<St, kTX, kTY, NST>;
+    auto kern = pair_step<St, kTX, TY, NST>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
     if (e != cudaSuccess) return e;
-    const Split s = split(g, sms);
+    const Split s = split(g, (int)eb, sms);
     const PairWork w{(int)s.tiles_x, (int)s.tiles, (int)s.items, s.zc, work};
     const int grid = s.items < sms ? (int)s.items : sms;
     kern<<<grid, S::THREADS, S::SMEM, st>>>(map, pair_slots(out, g, (int)eb), g, (float)p.inv_tau, (float)p.lid_u,
@@ -111,20 +114,20 @@ cudaError_t launch(const void* in, void* out, const Grid& g, const Params& p, in
 
 bool pair_step_pays(int storage, const Grid& g)
 {
-    if (storage < 1 || storage > 3) return false;  // F16SR: its dither makes the pair 4 % slower to 4 % faster
+    if (storage < 1 || storage > 4) return false;
     const int eb = storage_elem_bytes(storage);
     // the copies' 16-byte alignment, 32-bit offsets into a slot, 32-bit item numbers
     if (!default_layout(g, eb) || (unsigned long long)g.S * eb >= (1ull << 32) || !encode_fn()) return false;
     const int sms = sm_count();
     if (sms < 1) return false;
-    const Split s = split(g, sms);
+    const Split s = split(g, eb, sms);
     if (s.items > (1ll << 30)) return false;
     // Measured on GB300, microseconds: a plane of a block, and the separate
     // kernels' cells per microsecond from memory and, while the state fits L2,
     // from there (the pair kernel works on two arrays and so never does).
-    static const double plane[4] = {0, 1.80, 1.45, 1.43};
-    static const double rate[4] = {0, 43000, 80000, 80000};
-    static const double rate_l2[4] = {0, 54000, 75000, 75000};
+    static const double plane[5] = {0, 1.80, 1.70, 1.67, 1.96};
+    static const double rate[5] = {0, 43000, 80000, 80000, 79000};
+    static const double rate_l2[5] = {0, 54000, 75000, 75000, 70000};
     const double state = (double)Q * (double)g.S * eb;
     const double cells = (double)g.nx * g.ny * g.nz;
     const double separate = 2.0 * cells / (state < 100e6 ? rate_l2 : rate)[storage];
@@ -139,6 +142,7 @@ cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid&
     case 1: return launch<F32>(in, out, g, p, lid_y, work, err, st);
     case 2: return launch<F16S>(in, out, g, p, lid_y, work, err, st);
     case 3: return launch<BF16S>(in, out, g, p, lid_y, work, err, st);
+    case 4: return launch<F16SR>(in, out, g, p, lid_y, work, err, st);
     default: return cudaErrorInvalidValue;
     }
 }

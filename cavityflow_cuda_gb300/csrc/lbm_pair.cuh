@@ -33,9 +33,10 @@
 //
 // Measured on GB300 at 384^3 (ms a pair, separate kernels -> this one): FP32
 // 2.58 -> 1.49 (76.2 GLUP/s; 93 % of the copy bandwidth for the bytes it moves,
-// 1.11x its array in and 1.0x out), BF16S 1.38 -> 1.12 and F16S 1.39 -> 1.13
-// (100 GLUP/s; issue slots and the FP32 pipe, not memory: 54 % of the former
-// are used with 20 warps a SM).
+// 1.11x its array in and 1.0x out), BF16S 1.38 -> 1.09 (104 GLUP/s), F16SR
+// 1.41 -> 1.28 (88.8 GLUP/s; its dither is a fifth of its instructions).  The
+// 16-bit storages are bound by issue slots and the FP32 pipe (54-60 % of the
+// slots used), not by memory.
 #pragma once
 
 #include <cstdint>
@@ -300,7 +301,7 @@ struct PairShape {
     // one word
     static constexpr int SEP = sizeof(bits) == 4 ? TX / 2 : 1;
     static_assert(NB % 32 == 0, "whole warps");
-    static_assert(2 * NST <= 15, "named barriers");
+    static_assert(1 + 2 * NST <= 15, "named barriers");
 };
 
 // Named barriers, as a producer and a consumer use them: `arrive` does not wait.
@@ -462,10 +463,13 @@ __device__ __forceinline__ void pair_alpha(const Grid& g, const float inv_tau, c
     bool work = false, both = false, lid = false, wall = false;
 #pragma unroll 1
     for (;;) {
-        if (!pair_wait(&full[stage], phase, limit_ns)) {  // reported; the block runs on to its end
-            atomicOr(err, 4);
+        // one warp looks for the copy's arrival, the others sleep in a barrier: 11 or 13 warps looking took
+        // issue slots from beta's (F16SR 1.276 ms a pair instead of 1.296 at 384^3)
+        if (tid < 32 && !pair_wait(&full[stage], phase, limit_ns)) {
+            atomicOr(err, 4);  // reported; the block runs on to its end
             limit_ns = 1000000;
         }
+        named_sync(1 + 2 * NST, S::NA);
         const int now = *(const volatile int*)&item_of[stage];
         ++p;
         if (now != item) {  // another tile's first plane

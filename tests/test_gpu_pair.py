@@ -30,14 +30,15 @@ def _state(n, seed):
     return w[:, None, None, None] * (np.float32(0.98) + np.float32(0.04) * noise)
 
 
-# One cell beyond whole tiles of 64 x 8 and beyond whole z chunks (129 is too narrow for the pair kernel to pay, 449
-# is not); whole tiles; one tile less a cell; larger, where it pays for every storage it serves.
+# One cell beyond whole tiles of 64 x 8 (64 x 10) and beyond whole z chunks (129 is too narrow for the pair kernel to pay, 449
+# is not); whole tiles; one tile less a cell; larger, where it pays for the storages that round to nearest; larger
+# still for the stochastic one.
 SHAPES = [((129, 121, 131), "injection"), ((449, 121, 131), "injection"), ((192, 128, 97), "wall"),
           ((383, 63, 90), "injection"), ((320, 257, 249), "injection")]
 
 
-@pytest.mark.parametrize("storage", ["f32", "f16s", "bf16s"])
-@pytest.mark.parametrize("n,lid", SHAPES)
+@pytest.mark.parametrize("storage,n,lid", [(st, *shape) for shape in SHAPES for st in ("f32", "f16s", "bf16s")] +
+                         [("f16sr", (448, 383, 201), "wall")])
 def test_pairs_match_single_steps(gpu, oracle, storage, n, lid):
     from cavityflow_cuda_gb300 import kernel_launches
 
