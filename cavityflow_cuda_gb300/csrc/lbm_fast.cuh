@@ -114,6 +114,39 @@ __device__ __forceinline__ B shfl_down_bits(B v, int d)
     else return __shfl_down_sync(0xffffffffu, v, d);
 }
 
+// Programmatic dependent launch: a step kernel waits for the previous one's
+// results before it touches the populations, and lets the next one's blocks be
+// scheduled before it is complete.  A grid of more blocks than the chip holds
+// does so at once: the next step's blocks fill the SMs that its last wave
+// leaves.  A smaller grid does so when its blocks are done storing: earlier, the
+// next step's waiting blocks would hold the places that spread its own over the
+// SMs.  Graph-replayed steps, before -> now (late / at once), us: 32^3 FP32 2.18
+// -> 1.96 / 2.87, 48^3 3.28 -> 2.95 / 3.36, 96^3 16.26 -> 16.34 / 16.00, 128^3
+// F16SR 29.83 -> 30.19 / 29.54.  Without the launch attribute (launch_step) both
+// instructions do nothing.
+__device__ __forceinline__ void wait_previous_step() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_step() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <int BLOCK>
+__device__ __forceinline__ bool fills_chip()
+{
+    return gridDim.x * gridDim.y > 152u * 512u / (unsigned)BLOCK;
+}
+
+template <class Kernel, class... Args>
+cudaError_t launch_step(Kernel kern, dim3 grid, int block, cudaStream_t st, Args... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // The group of CPT cells a thread owns: group gi of row y of plane z.  An
 // inactive thread (past the end) carries a valid group (it reads, never
 // writes).
@@ -188,10 +221,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) alpha_fast(typename St::bits* __r
                                                           const uint32_t step_off, const FastDiv divG,
                                                           const int z_base)
 {
+    if (fills_chip<BLOCK>()) allow_next_step();
     const int G = (g.nx + CPT - 1) / CPT;
-    alpha_cells<St, CPT>(dd, g, inv_tau, lid_u, lid_y, wall_y,
-                         cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1),
-                         step_of<St>(step_base, step_off));
+    const Cells c = cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1);
+    wait_previous_step();
+    alpha_cells<St, CPT>(dd, g, inv_tau, lid_u, lid_y, wall_y, c, step_of<St>(step_base, step_off));
+    if (!fills_chip<BLOCK>()) allow_next_step();
 }
 
 // Beta step of the CPT cells of group `c`.  All 32 lanes of the warp must
@@ -630,10 +665,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) beta_fast_pk(typename St::bits* _
                                                             const uint32_t step_off, const FastDiv divG,
                                                             const int z_base)
 {
+    if (fills_chip<BLOCK>()) allow_next_step();
     const int G = (g.nx + CPT - 1) / CPT;
-    beta_cells_pk<St, CPT, kVec>(dd, g, inv_tau, lid_u, lid_y, wall_y,
-                                 cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1),
-                                 step_of<St>(step_base, step_off));
+    const Cells c = cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1);
+    wait_previous_step();
+    beta_cells_pk<St, CPT, kVec>(dd, g, inv_tau, lid_u, lid_y, wall_y, c, step_of<St>(step_base, step_off));
+    if (!fills_chip<BLOCK>()) allow_next_step();
 }
 
 template <class St, int CPT, int BLOCK, int MINB>
@@ -645,10 +682,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) beta_fast_direct(typename St::bit
                                                                 const uint32_t step_off, const FastDiv divG,
                                                                 const int z_base)
 {
+    if (fills_chip<BLOCK>()) allow_next_step();
     const int G = (g.nx + CPT - 1) / CPT;
-    beta_cells_direct<St, CPT>(dd, g, inv_tau, lid_u, lid_y, wall_y,
-                               cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1),
-                               step_of<St>(step_base, step_off));
+    const Cells c = cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1);
+    wait_previous_step();
+    beta_cells_direct<St, CPT>(dd, g, inv_tau, lid_u, lid_y, wall_y, c, step_of<St>(step_base, step_off));
+    if (!fills_chip<BLOCK>()) allow_next_step();
 }
 
 // Beta step with the neighbour exchange done block-wide: inside a warp by
@@ -820,11 +859,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) beta_fast_blk(typename St::bits* 
                                                              const uint32_t step_off, const FastDiv divG,
                                                              const int z_base)
 {
+    if (fills_chip<BLOCK>()) allow_next_step();
     const int G = (g.nx + CPT - 1) / CPT;
-    beta_cells_blk<St, CPT, BLOCK>(
-        dd, g, inv_tau, lid_u, lid_y, wall_y,
-        cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1),
-        step_of<St>(step_base, step_off));
+    const Cells c = cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1);
+    wait_previous_step();
+    beta_cells_blk<St, CPT, BLOCK>(dd, g, inv_tau, lid_u, lid_y, wall_y, c, step_of<St>(step_base, step_off));
+    if (!fills_chip<BLOCK>()) allow_next_step();
 }
 
 template <class St, int CPT, int BLOCK, int MINB>
@@ -836,10 +876,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) beta_fast(typename St::bits* __re
                                                          const uint32_t step_off, const FastDiv divG,
                                                          const int z_base)
 {
+    if (fills_chip<BLOCK>()) allow_next_step();
     const int G = (g.nx + CPT - 1) / CPT;
-    beta_cells<St, CPT>(dd, g, inv_tau, lid_u, lid_y, wall_y,
-                        cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1),
-                        step_of<St>(step_base, step_off));
+    const Cells c = cells_of_plane(g, G, divG, blockIdx.x * BLOCK + threadIdx.x, z_base + (int)blockIdx.y + 1);
+    wait_previous_step();
+    beta_cells<St, CPT>(dd, g, inv_tau, lid_u, lid_y, wall_y, c, step_of<St>(step_base, step_off));
+    if (!fills_chip<BLOCK>()) allow_next_step();
 }
 
 // Cells per thread of a kernel shape for storage St (at least one).
@@ -867,11 +909,12 @@ cudaError_t launch_fast_variant(bool alpha, void* dd, const Grid& g, const Param
         const unsigned bx = (unsigned)((per_plane + block - 1) / block);
         for (int z0 = 0; z0 < g.nz; z0 += kMaxPlanes) {
             const int planes = g.nz - z0 < kMaxPlanes ? g.nz - z0 : kMaxPlanes;
-            kern<<<dim3(bx, (unsigned)planes), block, 0, st>>>(d, g, T(p.inv_tau), T(p.lid_u), lid_y, p.wall_y,
-                                                               p.step_base, p.step_off, divG, z0);
+            const cudaError_t e = launch_step(kern, dim3(bx, (unsigned)planes), block, st, d, g, T(p.inv_tau), T(p.lid_u),
+                                              lid_y, p.wall_y, p.step_base, p.step_off, divG, z0);
+            if (e != cudaSuccess) return e;
             if (z0 > 0) add_launches(1);
         }
-        return cudaGetLastError();
+        return cudaSuccess;
     };
     if (alpha) {
         constexpr KernelShape k = fv.alpha;
@@ -996,6 +1039,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_step(typename St::bits* __r
     constexpr int kChunks = (int)(sizeof(BatchDomain) / 16);
     static_assert(kChunks <= BLOCK, "one thread per descriptor chunk");
     __shared__ BatchDomain desc[2];
+    wait_previous_step();
+    allow_next_step();  // the next step's blocks take the places of those that run out of virtual blocks
     const long long stride = gridDim.x;
     long long vb = blockIdx.x;
     if (vb >= vblocks) return;
@@ -1045,9 +1090,8 @@ cudaError_t launch_batch_kernel(const BatchArgs& a, cudaStream_t st)
     long long grid = (long long)(per_sm > 0 ? per_sm : 1) * sms;
     if (grid > a.vblocks) grid = a.vblocks;
     if (grid < 1) return cudaSuccess;
-    kern<<<(int)grid, k.block, 0, st>>>(static_cast<typename St::bits*>(a.pool), a.doms, a.vb_dom, a.vblocks,
-                                        a.step_base, a.step_off);
-    return cudaGetLastError();
+    return launch_step(kern, dim3((unsigned)grid), k.block, st, static_cast<typename St::bits*>(a.pool), a.doms, a.vb_dom,
+                       a.vblocks, a.step_base, a.step_off);
 }
 
 template <class St, int VARIANT>
