@@ -104,13 +104,18 @@ int lbm_detail::default_batch_variant(int storage)
     }
 }
 
-int lbm_detail::default_variant(int storage)
+// The 16-bit storages' 8- and 4-cell threads are long serial chains: on domains
+// that do not fill the chip with them fewer cells a thread are faster (us a step
+// in a replayed graph, F16SR: 32^3 variant 20 3.95, 6 2.67; 64^3 20 6.23, 6 5.67,
+// 8 5.07; 96^3 20 13.5, 8 12.6, 23 12.5; 112^3 20 19.1, 8 18.8, 23 18.0; 128^3 20
+// 30.2, 23 30.0, 8 34.5; BF16S alike).
+int lbm_detail::default_variant(int storage, long long cells)
 {
     switch (storage) {
-    case LBM_STORAGE_F32: return 13;
-    case LBM_STORAGE_F16S: return 20;
-    case LBM_STORAGE_BF16S: return 20;
-    case LBM_STORAGE_F16SR: return 20;
+    case LBM_STORAGE_F16S:
+    case LBM_STORAGE_BF16S:
+    case LBM_STORAGE_F16SR:
+        return cells < 170000 ? 6 : cells < 1100000 ? 8 : cells < 1900000 ? 23 : 20;
     default: return 13;
     }
 }
@@ -520,7 +525,9 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
         return fail(LBM_ERR_INVALID_ARGUMENT, "fast_variant %d not in [0, %d]", prm->fast_variant,
                     lbm::kFastVariantCount);
     }
-    s->variant = prm->fast_variant == 0 ? default_variant(s->storage) : prm->fast_variant - 1;
+    s->variant = prm->fast_variant == 0
+                     ? default_variant(s->storage, (long long)s->g.nx * s->g.ny * s->g.nz)
+                     : prm->fast_variant - 1;
     s->pairs = prm->fast_variant == 0;
     s->fma = prm->fused_multiply_add == 1;
     s->lid_mode = prm->lid_mode;
