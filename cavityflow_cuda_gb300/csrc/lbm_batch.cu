@@ -39,6 +39,7 @@ struct lbm_batch {
     void* pool = nullptr;
     size_t pool_bytes = 0;
     std::vector<lbm_solver*> views;
+    PackBuffer pack;  // the domains' getters take turns with it
     std::vector<lbm::BatchDomain> table;
     lbm::BatchDomain* dtable = nullptr;
     uint32_t* step_words = nullptr;  // [0] first step of a graph replay, [1] zero
@@ -133,6 +134,7 @@ void free_batch(lbm_batch* b)
     for (int kind = 0; kind < 2; ++kind)
         if (b->vb_map[kind]) cudaFree(b->vb_map[kind]);
     if (b->step_words) cudaFree(b->step_words);
+    free_pack(b->pack);
     if (b->pool) cudaFree(b->pool);
     delete b;
 }
@@ -223,6 +225,7 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
                               lbm::kPackedX1Align);
         if (r) return bail(r);
         v->batch = b;
+        v->batch_pack = &b->pack;
         b->views.push_back(v);
         r = lbm_set_driven_cavity(v);
         if (r) return bail(r);
@@ -259,6 +262,7 @@ int lbm_batch_get_info(const lbm_batch* b, lbm_batch_info* info)
     int64_t bytes = (int64_t)b->pool_bytes + (int64_t)(b->table.size() * sizeof(lbm::BatchDomain)) +
                     (int64_t)((b->vb_cap[0] + b->vb_cap[1]) * (long long)sizeof(int));
     for (const lbm_solver* v : b->views) bytes += v->device_bytes;
+    bytes += (int64_t)b->pack.bytes;
     info->device_bytes = bytes;
     return LBM_OK;
 }

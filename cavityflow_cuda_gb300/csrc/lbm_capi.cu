@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -285,25 +286,119 @@ bool ensure_pairs(lbm_solver* s, cudaStream_t st)
     return true;
 }
 
-int ensure_macros(lbm_solver* s)
+constexpr size_t kPackBytes = (size_t)96 << 20;  // larger calls copy at the link's rate without packing
+
+// What a solver's packing buffer is made for: density and velocity of the
+// interior, its populations if they are few.
+size_t pack_capacity(const lbm_solver* s)
 {
+    const size_t cells = (size_t)s->g.nx * s->g.ny * s->g.nz * value_bytes(s->storage);
+    if (4 * cells > kPackBytes) return 0;
+    return lbm::Q * cells <= ((size_t)24 << 20) ? lbm::Q * cells : 3 * cells;
+}
+
+// Computes the macroscopic fields on the default stream if a step has been taken
+// since (`computed`); check_macros follows once that stream is idle.
+int ensure_macros(lbm_solver* s, bool& computed)
+{
+    computed = false;
     CK(cudaSetDevice(s->device), "cudaSetDevice");
     if (!s->macros) {
-        const size_t bytes = (size_t)4 * s->g.cells() * value_bytes(s->storage);
-        CK(alloc_or_drop_pairs(s, &s->macros, bytes), "cudaMalloc macros");
+        // the packing buffer in the same allocation, where it fits
+        const size_t bytes = ((size_t)4 * s->g.cells() * value_bytes(s->storage) + 255) / 256 * 256;
+        std::lock_guard<std::mutex> lock(s->pack.mutex);
+        const size_t tail = s->batch_pack || s->pack.p ? 0 : pack_capacity(s);
+        if (tail > 0 && cudaEventCreateWithFlags(&s->pack.idle, cudaEventDisableTiming) == cudaSuccess &&
+            cudaMalloc(&s->macros, bytes + tail) == cudaSuccess) {
+            s->pack.p = static_cast<char*>(s->macros) + bytes;
+            s->pack.bytes = tail;
+            s->pack.owned = false;
+        } else {
+            cudaGetLastError();
+            s->macros = nullptr;
+            CK(alloc_or_drop_pairs(s, &s->macros, bytes), "cudaMalloc macros");
+        }
         s->device_bytes += (int64_t)bytes;
         s->macros_fresh = false;
     }
     if (!s->macros_fresh) {
         CK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
-        if (int r = check_kernel_flag(s)) return r;
-        CK(lbm::launch_macros(s->storage, s->dd, s->flags, s->g, s->last_alpha, s->p.lid_u, s->macros, 0),
+        CK(lbm::launch_macros(s->storage, s->dd, s->flags, s->g, s->last_alpha, s->p.lid_u, s->macros, err_flag(s),
+                              reinterpret_cast<int*>(s->host_out + 4), 0),
            "compute_macros launch");
-        CK(cudaDeviceSynchronize(), "compute_macros");
         s->macros_fresh = true;
+        computed = true;
     }
     return LBM_OK;
 }
+
+// After the default stream is idle: whether the step kernels behind the fields
+// that ensure_macros computed (`computed`) gave up a wait.
+int check_macros(lbm_solver* s, bool computed)
+{
+    if (!computed || *reinterpret_cast<volatile int*>(s->host_out + 4) == 0) return LBM_OK;
+    s->macros_fresh = false;
+    return check_kernel_flag(s);
+}
+
+// The solver's (or its batch's) buffer for one call's packed values, taken for
+// the life of this object: calls of several threads take turns, and the work of
+// a call on another stream waits for the previous call's (the event).  Null
+// where the call is too large for it to matter, the stream is capturing or
+// there is no memory: the caller then copies row by row.
+class Packed {
+public:
+    Packed(lbm_solver* s, size_t bytes, cudaStream_t st) : b_(s->batch_pack ? *s->batch_pack : s->pack), st_(st)
+    {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (bytes > kPackBytes) return;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        if (capture != cudaStreamCaptureStatusNone) return;
+        lock_ = std::unique_lock<std::mutex>(b_.mutex);
+        if (b_.bytes < bytes && !grow(s, bytes)) return;
+        if (cudaStreamWaitEvent(st, b_.idle, 0) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        p_ = b_.p;
+    }
+    ~Packed()
+    {
+        if (p_ && cudaEventRecord(b_.idle, st_) != cudaSuccess) cudaGetLastError();
+    }
+    Packed(const Packed&) = delete;
+    Packed& operator=(const Packed&) = delete;
+    void* get() const { return p_; }
+
+private:
+    bool grow(lbm_solver* s, size_t bytes)
+    {
+        const size_t want = std::max(bytes, std::min(kPackBytes, pack_capacity(s)));
+        if (!b_.idle && cudaEventCreateWithFlags(&b_.idle, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            b_.idle = nullptr;
+            return false;
+        }
+        if (b_.p && b_.owned) cudaFree(b_.p);  // waits for the device
+        b_.p = nullptr;
+        b_.bytes = 0;
+        b_.owned = true;
+        if (cudaMalloc(&b_.p, want) != cudaSuccess) {
+            cudaGetLastError();
+            b_.p = nullptr;
+            return false;
+        }
+        b_.bytes = want;
+        return true;
+    }
+    lbm_detail::PackBuffer& b_;
+    cudaStream_t st_;
+    std::unique_lock<std::mutex> lock_;
+    void* p_ = nullptr;
+};
 
 // Synchronous cuboid copy between a compact reference-layout device array
 // (x extent nx+2) and a packed host buffer.
@@ -552,7 +647,7 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
         return bail(cuda_fail(e, "cudaMemset counters"));
     s->p.step_base = step_words(s) + 1;  // direct launches: step = step_off
     s->p.step_off = 0;
-    if ((e = cudaMallocHost(&s->host_out, 4 * sizeof(double))) != cudaSuccess)
+    if ((e = cudaMallocHost(&s->host_out, 5 * sizeof(double))) != cudaSuccess)
         return bail(cuda_fail(e, "cudaMallocHost"));
     if ((e = cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking)) != cudaSuccess)
         return bail(cuda_fail(e, "cudaStreamCreate"));
@@ -572,6 +667,15 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
     return LBM_OK;
 }
 
+void lbm_detail::free_pack(PackBuffer& b)
+{
+    if (b.p && b.owned) cudaFree(b.p);
+    if (b.idle) cudaEventDestroy(b.idle);
+    b.p = nullptr;
+    b.bytes = 0;
+    b.idle = nullptr;
+}
+
 void lbm_detail::destroy_solver(lbm_solver* s)
 {
     if (!s) return;
@@ -581,6 +685,7 @@ void lbm_detail::destroy_solver(lbm_solver* s)
     if (s->capture_stream) cudaStreamDestroy(s->capture_stream);
     if (s->dd && s->owns_dd) cudaFree(s->dd);
     if (s->dd2) cudaFree(s->dd2);
+    free_pack(s->pack);
     if (s->flags) cudaFree(s->flags);
     if (s->macros) cudaFree(s->macros);
     if (s->scratch) cudaFree(s->scratch);
@@ -625,7 +730,7 @@ int lbm_get_info(const lbm_solver* s, lbm_info* info)
                                                                             : 0;
     info->row_pitch = s->g.P;
     info->slot_stride = s->g.S;
-    info->device_bytes = s->device_bytes;
+    info->device_bytes = s->device_bytes + (int64_t)s->pack.bytes;
     info->lid_mode = s->lid_mode;
     info->moving_wall = s->p.wall_y > 0 ? 1 : 0;
     info->x1_column = s->g.xoff + 1;
@@ -888,6 +993,15 @@ int lbm_get_density_distributions(lbm_solver* s, const int32_t origin[3], const 
     CK(cudaSetDevice(s->device), "cudaSetDevice");
     const size_t cells = (size_t)n.x * n.y * n.z;
     char* h = static_cast<char*>(host);
+    {
+        const size_t bytes = (size_t)lbm::Q * cells * (size_t)value_bytes(s->storage);
+        Packed packed(s, bytes, st);
+        if (packed.get()) {
+            CK(lbm::launch_pack_slots(s->storage, s->dd, s->g, o, n, packed.get(), st), "pack_slots launch");
+            CK(cudaMemcpyAsync(h, packed.get(), bytes, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+            return LBM_OK;
+        }
+    }
     if (s->storage <= LBM_STORAGE_F32) {
         for (int k = 0; k < lbm::Q; ++k)
             CK(copy_slot(s, k, o, n, h + (size_t)k * cells * elem_bytes(s->storage), true, st), "cudaMemcpy3DAsync");
@@ -986,15 +1100,25 @@ static int macro_copy(lbm_solver* s, const int32_t* origin, const int32_t* size,
     if (!host) return fail(LBM_ERR_INVALID_ARGUMENT, "host buffer is NULL");
     int3 o, n;
     if (int r = resolve_cuboid(s, origin, size, o, n)) return r;
-    if (int r = ensure_macros(s)) return r;
+    bool computed = false;
+    if (int r = ensure_macros(s, computed)) return r;
     const size_t vb = (size_t)value_bytes(s->storage);
     const size_t cells = (size_t)n.x * n.y * n.z;
-    for (int c = 0; c < count; ++c) {
-        char* dev = static_cast<char*>(s->macros) + (size_t)(first + c) * s->g.cells() * vb;
-        char* h = static_cast<char*>(host) + (size_t)c * cells * vb;
-        CK(copy_compact(dev, vb, s->g, o, n, h, to_host), "cudaMemcpy3D macros");
+    char* const field = static_cast<char*>(s->macros) + (size_t)first * s->g.cells() * vb;
+    if (to_host) {
+        Packed packed(s, cells * vb * (size_t)count, 0);
+        if (packed.get()) {
+            CK(lbm::launch_pack_compact((int)vb, field, count, s->g, o, n, packed.get(), 0), "pack_compact launch");
+            CK(cudaMemcpy(host, packed.get(), cells * vb * (size_t)count, cudaMemcpyDeviceToHost), "cudaMemcpy macros");
+            return check_macros(s, computed);
+        }
     }
-    return LBM_OK;
+    for (int c = 0; c < count; ++c) {
+        char* h = static_cast<char*>(host) + (size_t)c * cells * vb;
+        CK(copy_compact(field + (size_t)c * s->g.cells() * vb, vb, s->g, o, n, h, to_host), "cudaMemcpy3D macros");
+    }
+    if (computed) CK(cudaStreamSynchronize(0), "cudaStreamSynchronize");
+    return check_macros(s, computed);
 }
 
 int lbm_get_velocities(lbm_solver* s, const int32_t origin[3], const int32_t size[3], void* host)

@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <exception>
+#include <mutex>
 #include <new>
 #include <cuda_runtime.h>
 
@@ -11,6 +12,21 @@
 #include "lbm_kernels.h"
 
 struct lbm_batch;
+
+namespace lbm_detail {
+
+// Device buffer in which the getters pack a call's values for one contiguous
+// copy to the host; `idle` is recorded behind the copy that last used it.
+struct PackBuffer {
+    std::mutex mutex;
+    cudaEvent_t idle = nullptr;
+    void* p = nullptr;
+    size_t bytes = 0;
+    bool owned = true;  // false: the end of the solver's macros array
+};
+void free_pack(PackBuffer& b);
+
+}  // namespace lbm_detail
 
 struct lbm_solver {
     lbm::Grid g{};
@@ -25,7 +41,7 @@ struct lbm_solver {
     double* scratch = nullptr;      // reduction partials (4 per block) + result (4)
     unsigned long long* counts = nullptr;  // cavity-flag check counters [0..1], kernel error flag [2],
                                            // work words of the pair kernel [3], step words [4] (see step_words)
-    double* host_out = nullptr;     // pinned, 4 doubles
+    double* host_out = nullptr;     // pinned: the reduction's 4 doubles, then the error flag of compute_macros
     float* staging = nullptr;       // 16-bit storage: one packed slot cuboid
     size_t staging_elems = 0;
     int64_t counter = 0;
@@ -35,6 +51,8 @@ struct lbm_solver {
     bool fma = false;               // FP64: fused multiply-adds in the vectorised steps
     int lid_mode = 0;               // LBM_LID_INJECTION or LBM_LID_MOVING_WALL; the wall moves
                                     // while p.wall_y > 0
+    lbm_detail::PackBuffer pack;    // the getters' packing buffer
+    lbm_detail::PackBuffer* batch_pack = nullptr;  // a batch domain's: shared by the batch
     void* dd2 = nullptr;            // lbm_run's second population array (ensure_pairs)
     bool pairs = true;              // lbm_run may take two steps a pass: no launch variant was asked for
     bool pairs_refused = false;     // no memory for dd2

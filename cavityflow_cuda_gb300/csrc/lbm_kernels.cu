@@ -209,9 +209,11 @@ __device__ __forceinline__ void post_populations(const typename St::bits* dd, co
 template <class St>
 __global__ void compute_macros(const typename St::bits* __restrict__ dd, const uint8_t* __restrict__ flags,
                                const Grid g, const bool last_alpha, const typename St::T lid_u,
-                               typename St::T* __restrict__ out)
+                               typename St::T* __restrict__ out, const int* __restrict__ err,
+                               int* __restrict__ host_err)
 {
     using T = typename St::T;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *host_err = *err;  // with the fields, so that it needs no copy of its own
     const long long n = g.cells();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
@@ -334,6 +336,41 @@ __global__ void reduce_final(const double* __restrict__ partials, int nblocks, d
         double s = 0.0;
         for (int b = 0; b < nblocks; ++b) s += partials[b * 4 + threadIdx.x];
         out[threadIdx.x] = s;
+    }
+}
+
+// A cuboid of `count` arrays in the compact reference layout, `stride` values
+// apart, packed x fastest one after the other; or of the 19 slots of the
+// populations (stride g.S, padded rows) with the weights added back to shifted
+// storage.  A warp walks rows, its lanes along x; one contiguous copy then takes
+// the result to the host, where a copy of its short rows one by one runs far
+// below the link (64^3 velocities: 58 us as three 3-D copies, 36 us packed).
+template <typename T>
+__global__ void __launch_bounds__(256) pack_compact(const T* __restrict__ src, const long long stride, const int count,
+                                                    const Grid g, const int3 o, const int3 s, T* __restrict__ out)
+{
+    const unsigned rows = (unsigned)(s.y * s.z), all = rows * (unsigned)count;
+    for (unsigned r = blockIdx.x * 8 + (threadIdx.x >> 5); r < all; r += gridDim.x * 8) {
+        const unsigned c = r / rows, rr = r - c * rows, z = rr / (unsigned)s.y, y = rr - z * (unsigned)s.y;
+        const T* p = src + c * stride + g.ref(o.x, o.y + (int)y, o.z + (int)z);
+        T* q = out + (long long)r * s.x;
+        for (int x = threadIdx.x & 31; x < s.x; x += 32) q[x] = p[x];
+    }
+}
+template <class St>
+__global__ void __launch_bounds__(256) pack_slots(const typename St::bits* __restrict__ dd, const Grid g, const int3 o,
+                                                  const int3 s, typename St::T* __restrict__ out)
+{
+    const unsigned rows = (unsigned)(s.y * s.z), all = rows * (unsigned)Q;
+    for (unsigned r = blockIdx.x * 8 + (threadIdx.x >> 5); r < all; r += gridDim.x * 8) {
+        const unsigned k = r / rows, rr = r - k * rows, z = rr / (unsigned)s.y, y = rr - z * (unsigned)s.y;
+        const typename St::bits* p = dd + k * g.S + g.idx(o.x, o.y + (int)y, o.z + (int)z);
+        typename St::T* q = out + (long long)r * s.x;
+        const float w = k == 18 ? weight<float>(18) : k < 4 || k >= 16 ? weight<float>(0) : weight<float>(4);
+        for (int x = threadIdx.x & 31; x < s.x; x += 32) {
+            const typename St::T v = St::load(p[x]);
+            q[x] = St::shifted ? v + (typename St::T)w : v;
+        }
     }
 }
 
@@ -585,14 +622,39 @@ cudaError_t launch_general_step(int storage, bool alpha, void* dd, const uint8_t
 }
 
 cudaError_t launch_macros(int storage, const void* dd, const uint8_t* flags, const Grid& g, bool last_alpha,
-                          double lid_u, void* out, cudaStream_t st)
+                          double lid_u, void* out, const int* err, int* host_err, cudaStream_t st)
 {
     count_launch();
     return with_storage(storage, [&](auto tag) {
         using St = decltype(tag);
         using T = typename St::T;
         compute_macros<St><<<grid_for(g.cells(), 256, 8192), 256, 0, st>>>(
-            static_cast<const typename St::bits*>(dd), flags, g, last_alpha, T(lid_u), static_cast<T*>(out));
+            static_cast<const typename St::bits*>(dd), flags, g, last_alpha, T(lid_u), static_cast<T*>(out), err, host_err);
+        return cudaGetLastError();
+    });
+}
+
+cudaError_t launch_pack_compact(int value_bytes, const void* src, int count, const Grid& g, int3 o, int3 s, void* out,
+                                cudaStream_t st)
+{
+    count_launch();
+    const int grid = grid_for((long long)s.y * s.z * count, 8, 4096);
+    if (value_bytes == 8)
+        pack_compact<double><<<grid, 256, 0, st>>>(static_cast<const double*>(src), g.cells(), count, g, o, s,
+                                                   static_cast<double*>(out));
+    else
+        pack_compact<float><<<grid, 256, 0, st>>>(static_cast<const float*>(src), g.cells(), count, g, o, s,
+                                                  static_cast<float*>(out));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pack_slots(int storage, const void* dd, const Grid& g, int3 o, int3 s, void* out, cudaStream_t st)
+{
+    count_launch();
+    return with_storage(storage, [&](auto tag) {
+        using St = decltype(tag);
+        pack_slots<St><<<grid_for((long long)s.y * s.z * Q, 8, 4096), 256, 0, st>>>(
+            static_cast<const typename St::bits*>(dd), g, o, s, static_cast<typename St::T*>(out));
         return cudaGetLastError();
     });
 }

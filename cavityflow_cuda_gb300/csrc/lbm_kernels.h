@@ -181,8 +181,15 @@ cudaError_t launch_tma_f16sr(bool alpha, void* dd, const Grid& g, const Params& 
                              int stages, int consumer_warps, int* err, cudaStream_t st);
 cudaError_t launch_general_step(int storage, bool alpha, void* dd, const uint8_t* flags, const Grid& g,
                                 const Params& p, int3 origin, int3 size, cudaStream_t st);
+// Also copies the kernels' error flag *err to *host_err (mapped host memory).
 cudaError_t launch_macros(int storage, const void* dd, const uint8_t* flags, const Grid& g, bool last_alpha,
-                          double lid_u, void* out, cudaStream_t st);
+                          double lid_u, void* out, const int* err, int* host_err, cudaStream_t st);
+// A cuboid of `count` compact reference-layout arrays (g.cells() values apart),
+// or of the 19 population slots as host values, packed x fastest; s.y * s.z * 19
+// must fit 31 bits.
+cudaError_t launch_pack_compact(int value_bytes, const void* src, int count, const Grid& g, int3 o, int3 s, void* out,
+                                cudaStream_t st);
+cudaError_t launch_pack_slots(int storage, const void* dd, const Grid& g, int3 o, int3 s, void* out, cudaStream_t st);
 // Interior density and velocity of a box cavity with the lid on y = ny, from
 // the geometry; packed x fastest (rho, jx, jy, jz planes); `out` may be
 // mapped host memory.
