@@ -504,30 +504,41 @@ __device__ __forceinline__ double relax_f64(double f, double e, double inv_tau)
     return f + (f64::exp_ok(d) ? f64::mul(inv_tau, d) : inv_tau * d);
 }
 
-// relax_pair; s and inv_tau exp_ok.  P + (-3 s) is P - 3 s.
+// relax_pair; s exp_ok or zero, P and inv_tau exp_ok.  P + (-3 s) is P - 3 s;
+// with s = +-0 both sums are P.
 __device__ __forceinline__ void relax_pair_f64(double& fp, double& fm, double w, double P, double s, double inv_tau)
 {
-    const double t = f64::mul4_5(f64::mul(s, s));
-    const double a = f64::mul3(s);
-    const double p = (P + a) + t, m = (P - a) + t;
+    double p = P, m = P;
+    if (!f64::is_zero(s)) {
+        const double t = f64::mul4_5(f64::mul(s, s));
+        const double a = f64::mul3(s);
+        p = (P + a) + t;
+        m = (P - a) + t;
+    }
     const bool ok = f64::exp_ok(p) && f64::exp_ok(m);
     fp = relax_f64(fp, ok ? f64::mul(w, p) : w * p, inv_tau);
     fm = relax_f64(fm, ok ? f64::mul(w, m) : w * m, inv_tau);
 }
+
+__device__ __forceinline__ double square_f64(double v) { return f64::is_zero(v) ? 0.0 : f64::mul(v, v); }
 
 __device__ __forceinline__ void collide_fluid_f64(double* f, double inv_tau)
 {
     double rho, vx, vy, vz;
     moments(f, rho, vx, vy, vz);
     const double xpy = vx + vy, xmy = vx - vy, xpz = vx + vz, xmz = vx - vz, ypz = vy + vz, ymz = vy - vz;
-    const bool ok = f64::exp_ok(vx) && f64::exp_ok(vy) && f64::exp_ok(vz) && f64::exp_ok(xpy) && f64::exp_ok(xmy) &&
-                    f64::exp_ok(xpz) && f64::exp_ok(xmz) && f64::exp_ok(ypz) && f64::exp_ok(ymz) && f64::exp_ok(inv_tau);
-    if (!ok) {
+    auto fits = [](double s) { return f64::exp_ok(s) || f64::is_zero(s); };
+    if (!(fits(vx) && fits(vy) && fits(vz) && fits(xpy) && fits(xmy) && fits(xpz) && fits(xmz) && fits(ypz) &&
+          fits(ymz) && f64::exp_ok(inv_tau))) {
         collide_fluid(f, inv_tau);
         return;
     }
-    const double vel2 = f64::mul(vx, vx) + f64::mul(vy, vy) + f64::mul(vz, vz);
-    const double P = rho - f64::mul1_5(vel2);
+    const double vel2 = square_f64(vx) + square_f64(vy) + square_f64(vz);
+    const double P = rho - (f64::is_zero(vel2) ? vel2 : f64::mul1_5(vel2));
+    if (!f64::exp_ok(P)) {
+        collide_fluid(f, inv_tau);
+        return;
+    }
     const double wa = 1.0 / 18.0, wd = 1.0 / 36.0;
     relax_pair_f64(f[0], f[1], wa, P, vx, inv_tau);
     relax_pair_f64(f[2], f[3], wa, P, vy, inv_tau);
@@ -538,7 +549,7 @@ __device__ __forceinline__ void collide_fluid_f64(double* f, double inv_tau)
     relax_pair_f64(f[12], f[13], wd, P, ypz, inv_tau);
     relax_pair_f64(f[14], f[15], wd, P, ymz, inv_tau);
     relax_pair_f64(f[16], f[17], wa, P, vz, inv_tau);
-    f[18] = relax_f64(f[18], f64::exp_ok(P) ? f64::mul(1.0 / 3.0, P) : (1.0 / 3.0) * P, inv_tau);
+    f[18] = relax_f64(f[18], f64::mul(1.0 / 3.0, P), inv_tau);
 }
 
 // Collision dispatch by storage: the reference's arithmetic for F64/F32, the

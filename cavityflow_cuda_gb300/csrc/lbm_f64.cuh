@@ -12,9 +12,9 @@
 // results, bit for bit.
 //
 // The integer products take operands well inside the normal range (exp_ok).
-// Cells outside it (a velocity component or sum that is zero, subnormal,
-// infinite or NaN: the fluid at rest, a plane of symmetry) take the plain
-// collision, and so does a direction pair whose equilibrium is out of range.
+// Zero velocities (the fluid at rest, planes of symmetry) need no product; a
+// cell with any other operand outside that range (subnormal, infinite, NaN)
+// takes the plain collision.
 #pragma once
 
 #include <cstdint>
