@@ -91,17 +91,19 @@ constexpr int kGraphPairs = 32;  // alpha/beta pairs per captured graph
 
 // Batch and server rows are packed for 8-byte vectors (kPackedX1Align), so
 // their variants use 8-byte (or narrower) vectors in both kernels.  On the
-// seeded 512-cavity workload the direct beta windows in two-warp blocks
-// (variant 13) are fastest for FP32, the packed 16-bit beta at <= 128
-// registers (22: the batch kernel's own state spills the 102-register
-// shape) for the 16-bit storages.
+// seeded workload (ms a pair of 64 / 512 cavities): FP32 the direct beta windows
+// in four-warp blocks (variant 14: 0.728 / 5.32; 13, two warps: 0.755 / 5.51; 17,
+// eight: 0.736 / 5.28, and behind 14 on 8 cavities), the 16-bit storages the
+// packed beta at <= 128 registers (22: the batch kernel's own state spills the
+// 102-register shape), FP64 the warp exchange (3: 6.71 of 64; 13: 6.98).
 int lbm_detail::default_batch_variant(int storage)
 {
     switch (storage) {
     case LBM_STORAGE_F16S:
     case LBM_STORAGE_BF16S:
     case LBM_STORAGE_F16SR: return 22;
-    default: return 13;
+    case LBM_STORAGE_F64: return 3;
+    default: return 14;
     }
 }
 

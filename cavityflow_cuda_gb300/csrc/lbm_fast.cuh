@@ -133,7 +133,7 @@ __device__ __forceinline__ bool fills_chip()
 }
 
 template <class Kernel, class... Args>
-cudaError_t launch_step(Kernel kern, dim3 grid, int block, cudaStream_t st, Args... args)
+cudaError_t launch_step(Kernel kern, dim3 grid, int block, cudaStream_t st, size_t smem, const Args&... args)
 {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -141,6 +141,7 @@ cudaError_t launch_step(Kernel kern, dim3 grid, int block, cudaStream_t st, Args
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
@@ -909,7 +910,7 @@ cudaError_t launch_fast_variant(bool alpha, void* dd, const Grid& g, const Param
         const unsigned bx = (unsigned)((per_plane + block - 1) / block);
         for (int z0 = 0; z0 < g.nz; z0 += kMaxPlanes) {
             const int planes = g.nz - z0 < kMaxPlanes ? g.nz - z0 : kMaxPlanes;
-            const cudaError_t e = launch_step(kern, dim3(bx, (unsigned)planes), block, st, d, g, T(p.inv_tau), T(p.lid_u),
+            const cudaError_t e = launch_step(kern, dim3(bx, (unsigned)planes), block, st, 0, d, g, T(p.inv_tau), T(p.lid_u),
                                               lid_y, p.wall_y, p.step_base, p.step_off, divG, z0);
             if (e != cudaSuccess) return e;
             if (z0 > 0) add_launches(1);
@@ -1090,7 +1091,7 @@ cudaError_t launch_batch_kernel(const BatchArgs& a, cudaStream_t st)
     long long grid = (long long)(per_sm > 0 ? per_sm : 1) * sms;
     if (grid > a.vblocks) grid = a.vblocks;
     if (grid < 1) return cudaSuccess;
-    return launch_step(kern, dim3((unsigned)grid), k.block, st, static_cast<typename St::bits*>(a.pool), a.doms, a.vb_dom,
+    return launch_step(kern, dim3((unsigned)grid), k.block, st, 0, static_cast<typename St::bits*>(a.pool), a.doms, a.vb_dom,
                        a.vblocks, a.step_base, a.step_off);
 }
 

@@ -105,9 +105,8 @@ cudaError_t launch(const void* in, void* out, const Grid& g, const Params& p, in
     const Split s = split(g, (int)eb, sms);
     const PairWork w{(int)s.tiles_x, (int)s.tiles, (int)s.items, s.zc, work};
     const int grid = s.items < sms ? (int)s.items : sms;
-    kern<<<grid, S::THREADS, S::SMEM, st>>>(map, pair_slots(out, g, (int)eb), g, (float)p.inv_tau, (float)p.lid_u,
-                                            lid_y, p.wall_y, p.step_base, p.step_off, w, err);
-    return cudaGetLastError();
+    return launch_step(kern, dim3((unsigned)grid), S::THREADS, st, S::SMEM, map, pair_slots(out, g, (int)eb), g,
+                       (float)p.inv_tau, (float)p.lid_u, lid_y, p.wall_y, p.step_base, p.step_off, w, err);
 }
 
 }  // namespace

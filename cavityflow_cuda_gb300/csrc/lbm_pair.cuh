@@ -397,6 +397,9 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const Grid& g,
     using S = PairShape<St, TX, TY, NST>;
     const bool lead = (threadIdx.x & 31) == 0;
     int stage = 0, used = 0, item = (int)blockIdx.x;
+    // `in`, `out` and the counters are the previous step's until it is complete; the other threads touch global memory
+    // only after this warp's first copy has arrived
+    wait_previous_step();
 #pragma unroll 1
     while (item < w.items) {
         const PairItem it = pair_item<TX, TY>(w, g, item);
@@ -648,6 +651,7 @@ __global__ void __launch_bounds__(PairShape<St, TX, TY, NST>::THREADS, 1)
         tma::fence_mbar_init();
     }
     __syncthreads();
+    allow_next_step();  // its blocks take the SMs that this one's leave
     const uint32_t step = step_of<St>(step_base, step_off);
     if (threadIdx.x < S::NA)
         pair_alpha<St, TX, TY, NST>(g, inv_tau, lid_u, lid_y, wall_y, w, step, smem, full, item_of, err);
