@@ -6,10 +6,12 @@
 // so the per-domain getters, setters and reductions of the single-domain ABI
 // apply unchanged.  A batch step is one launch of the persistent batch
 // kernel (lbm_fast.cuh) over the packed domain table; long runs replay a CUDA
-// graph of captured alpha/beta pairs.
+// graph of captured alpha/beta pairs, or (FP32, where it is faster) take two
+// steps in one pass between the pool and a second one (lbm_pair.cuh).
 #include <cmath>
 #include <cstring>
 #include <exception>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -42,7 +44,15 @@ struct lbm_batch {
     PackBuffer pack;  // the domains' getters take turns with it
     std::vector<lbm::BatchDomain> table;
     lbm::BatchDomain* dtable = nullptr;
-    uint32_t* step_words = nullptr;  // [0] first step of a graph replay, [1] zero
+    uint32_t* step_words = nullptr;  // [0] first step of a graph replay, [1] zero, [2..3] work words of the pair
+                                     // kernel, [4] kernel error flag
+    lbm::PairBatchPlan pair_plan;    // two steps a pass, between the pool and a second one (ensure_batch_pairs)
+    bool pair_planned = false;
+    bool pairs = true;               // no launch variant was asked for
+    bool pairs_refused = false;      // no memory for the second pool
+    void* pool2 = nullptr;
+    void* pair_image = nullptr;      // the plan's image
+    std::mutex pair_mutex;           // views may give the second pool up from several threads
     long long vblocks[2] = {0, 0};  // virtual blocks of the alpha and the beta kernel
     int* vb_map[2] = {nullptr, nullptr};  // domain of each virtual block, per kernel
     long long vb_cap[2] = {0, 0};
@@ -61,6 +71,53 @@ void drop_batch_graph(lbm_batch* b)
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
+}
+
+void free_batch_pairs(lbm_batch* b)
+{
+    if (b->pool2) cudaFree(b->pool2);
+    if (b->pair_image) cudaFree(b->pair_image);
+    b->pool2 = b->pair_image = nullptr;
+}
+
+// Whether lbm_batch_run takes two steps a pass on `st`: from the pool to the
+// second one and back, so that the state is always in the pool when a call
+// returns.  The second pool is allocated by the first run that can use it, if
+// it takes at most a quarter of the free memory: the batch could do without
+// it.  A capturing stream gets the separate kernels: the caller's graph must not
+// hold an array that the batch may give up.
+bool ensure_batch_pairs(lbm_batch* b, cudaStream_t st)
+{
+    if (!b->pairs || b->pairs_refused) return false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return false;
+    if (!b->pair_planned) {
+        try {
+            lbm::plan_pair_batch(b->storage, b->table.data(), (int)b->table.size(), b->pair_plan);
+        } catch (const std::bad_alloc&) {
+            b->pair_plan = lbm::PairBatchPlan{};
+        }
+        b->pair_planned = true;
+    }
+    if (b->pair_plan.items == 0) return false;
+    std::lock_guard<std::mutex> lock(b->pair_mutex);
+    if (b->pool2) return true;
+    size_t free_b = 0, total_b = 0;
+    const size_t image = b->pair_plan.image.size();
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || b->pool_bytes > free_b / 4 ||
+        cudaMalloc(&b->pool2, b->pool_bytes) != cudaSuccess || cudaMalloc(&b->pair_image, image) != cudaSuccess ||
+        !lbm::bind_pair_batch(b->storage, b->pool, b->pool2, b->pair_plan) ||
+        cudaMemcpyAsync(b->pair_image, b->pair_plan.image.data(), image, cudaMemcpyHostToDevice, st) != cudaSuccess) {
+        cudaGetLastError();
+        free_batch_pairs(b);
+        b->pairs_refused = true;
+        return false;
+    }
+    return true;
 }
 
 // Numbers the virtual blocks of the current variant, uploads the table and
@@ -135,11 +192,21 @@ void free_batch(lbm_batch* b)
         if (b->vb_map[kind]) cudaFree(b->vb_map[kind]);
     if (b->step_words) cudaFree(b->step_words);
     free_pack(b->pack);
+    free_batch_pairs(b);
     if (b->pool) cudaFree(b->pool);
     delete b;
 }
 
 }  // namespace
+
+bool lbm_detail::drop_batch_pairs(lbm_batch* b)
+{
+    std::lock_guard<std::mutex> lock(b->pair_mutex);
+    if (!b->pool2) return false;
+    free_batch_pairs(b);
+    b->pairs_refused = true;
+    return true;
+}
 
 extern "C" {
 
@@ -185,8 +252,8 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
     size_t elems = 0;
     b->table.resize((size_t)count);
     for (int i = 0; i < count; ++i) {
-        const lbm::Grid g =
-            lbm::make_grid(domains[i].size[0], domains[i].size[1], domains[i].size[2], eb, lbm::kPackedX1Align);
+        const lbm::Grid g = lbm::make_grid(domains[i].size[0], domains[i].size[1], domains[i].size[2], eb,
+                                           lbm::kPackedX1Align, lbm::batch_pitch_align(storage));
         offsets[(size_t)i] = elems;
         elems += (size_t)lbm::Q * g.S;  // S keeps every slot 256-byte aligned
         lbm::BatchDomain& d = b->table[(size_t)i];
@@ -205,8 +272,8 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc batch table"));
     e = cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
-    e = cudaMalloc(&b->step_words, 2 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(b->step_words, 0, 2 * sizeof(uint32_t));
+    e = cudaMalloc(&b->step_words, 5 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(b->step_words, 0, 5 * sizeof(uint32_t));
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc batch step words"));
 
     b->views.reserve((size_t)count);
@@ -222,10 +289,11 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
         p.fast_variant = b->variant + 1;
         lbm_solver* v = nullptr;
         int r = create_solver(&p, static_cast<char*>(b->pool) + offsets[(size_t)i] * (size_t)eb, &v,
-                              lbm::kPackedX1Align);
+                              lbm::kPackedX1Align, lbm::batch_pitch_align(storage));
         if (r) return bail(r);
         v->batch = b;
         v->batch_pack = &b->pack;
+        v->batch_err = reinterpret_cast<int*>(b->step_words + 4);
         b->views.push_back(v);
         r = lbm_set_driven_cavity(v);
         if (r) return bail(r);
@@ -263,6 +331,7 @@ int lbm_batch_get_info(const lbm_batch* b, lbm_batch_info* info)
                     (int64_t)((b->vb_cap[0] + b->vb_cap[1]) * (long long)sizeof(int));
     for (const lbm_solver* v : b->views) bytes += v->device_bytes;
     bytes += (int64_t)b->pack.bytes;
+    if (b->pool2) bytes += (int64_t)(b->pool_bytes + b->pair_plan.image.size());
     info->device_bytes = bytes;
     return LBM_OK;
 }
@@ -296,6 +365,18 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
     if (left > 0 && b->last_alpha) {
         if ((r = one(false))) return r;
         --left;
+    }
+    if (left >= 4 && ensure_batch_pairs(b, st)) {
+        int* const work = reinterpret_cast<int*>(b->step_words + 2);
+        int* const err = reinterpret_cast<int*>(b->step_words + 4);
+        for (; left >= 4; left -= 4)
+            for (const bool back : {false, true}) {
+                CK(lbm::launch_pair_batch(b->storage, b->pair_plan, b->pair_image, back, back ? b->pool : b->pool2,
+                                          b->step_words + 1, (uint32_t)b->counter, work, err, st),
+                   "batch pair step launch");
+                b->counter += 2;
+                b->last_alpha = false;
+            }
     }
     const int64_t per_graph = 2 * kBatchGraphPairs;
     if (left >= per_graph) {
@@ -345,6 +426,7 @@ int lbm_batch_set_fast_variant(lbm_batch* b, int32_t variant)
     if (!b->views.empty() && !lbm::fast_variant_fits(b->storage, variant, b->views[0]->g))
         return fail(LBM_ERR_UNSUPPORTED, "variant %d's vectors do not fit the batch's packed rows", variant);
     CK(cudaSetDevice(b->device), "cudaSetDevice");
+    b->pairs = false;  // every step with the variant asked for
     b->variant = variant;
     for (lbm_solver* v : b->views) v->variant = variant;
     return build_table(b);
@@ -357,7 +439,12 @@ int lbm_batch_autotune(lbm_batch* b, int32_t pairs, int32_t* best, float* ms_per
     CK(cudaSetDevice(b->device), "cudaSetDevice");
     CK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     void* saved = nullptr;
-    CK(cudaMalloc(&saved, b->pool_bytes), "cudaMalloc autotune snapshot");
+    cudaError_t es = cudaMalloc(&saved, b->pool_bytes);
+    if (es == cudaErrorMemoryAllocation && drop_batch_pairs(b)) {
+        cudaGetLastError();
+        es = cudaMalloc(&saved, b->pool_bytes);
+    }
+    CK(es, "cudaMalloc autotune snapshot");
     cudaStream_t st = b->capture_stream;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     const int start_variant = b->variant;

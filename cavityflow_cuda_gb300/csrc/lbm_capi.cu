@@ -132,7 +132,10 @@ namespace {
 
 
 
-int* lbm_detail::err_flag(lbm_solver* s) { return reinterpret_cast<int*>(s->counts + 2); }
+int* lbm_detail::err_flag(lbm_solver* s)
+{
+    return s->batch_err ? s->batch_err : reinterpret_cast<int*>(s->counts + 2);
+}
 uint32_t* lbm_detail::step_words(lbm_solver* s) { return reinterpret_cast<uint32_t*>(s->counts + 4); }
 
 // Reads and clears the kernels' timeout flag after the device is idle.
@@ -246,7 +249,8 @@ void drop_pairs(lbm_solver* s)
     s->device_bytes -= (int64_t)((size_t)lbm::Q * s->g.S * elem_bytes(s->storage));
 }
 
-// cudaMalloc that gives up lbm_run's second population array rather than fail.
+// cudaMalloc that gives up the second population array of lbm_run (or of the
+// batch's runs) rather than fail.
 cudaError_t alloc_or_drop_pairs(lbm_solver* s, void** p, size_t bytes)
 {
     cudaError_t e = cudaMalloc(p, bytes);
@@ -254,6 +258,9 @@ cudaError_t alloc_or_drop_pairs(lbm_solver* s, void** p, size_t bytes)
         cudaGetLastError();
         drop_pairs(s);
         s->pairs_refused = true;
+        e = cudaMalloc(p, bytes);
+    } else if (e == cudaErrorMemoryAllocation && s->batch && drop_batch_pairs(s->batch)) {
+        cudaGetLastError();
         e = cudaMalloc(p, bytes);
     }
     return e;
@@ -577,7 +584,8 @@ int lbm_create(const lbm_params* prm, lbm_solver** out)
 
 }  // extern "C"
 
-int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solver** out, int x1_align)
+int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solver** out, int x1_align,
+                              int pitch_align)
 {
     if (!prm || !out) return fail(LBM_ERR_INVALID_ARGUMENT, "NULL argument");
     *out = nullptr;
@@ -610,7 +618,8 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
     if (!s) return fail(LBM_ERR_OUT_OF_MEMORY, "host allocation failed");
     s->storage = prm->storage;
     s->device = prm->device;
-    s->g = lbm::make_grid(prm->size[0], prm->size[1], prm->size[2], elem_bytes(prm->storage), x1_align);
+    s->g = lbm::make_grid(prm->size[0], prm->size[1], prm->size[2], elem_bytes(prm->storage), x1_align,
+                          pitch_align);
     s->p.inv_tau = prm->inv_tau;
     s->p.lid_u = prm->lid_velocity;
     s->p.gx = prm->gravity[0];

@@ -97,7 +97,7 @@ struct Grid {
 };
 
 // x1_align: byte alignment of x = 1, 32 (the default layout), 16 or 8.
-inline Grid make_grid(int nx, int ny, int nz, int elem_bytes, int x1_align = 32)
+inline Grid make_grid(int nx, int ny, int nz, int elem_bytes, int x1_align = 32, int pitch_align = 0)
 {
     Grid g;
     g.nx = nx; g.ny = ny; g.nz = nz;
@@ -106,7 +106,8 @@ inline Grid make_grid(int nx, int ny, int nz, int elem_bytes, int x1_align = 32)
     g.xoff = sector - 1;
     g.G = (nx + g.V - 1) / g.V;
     const long long need = (long long)g.xoff + (long long)g.G * g.V + 2;  // last scalar column + 1
-    g.P = (need + sector - 1) / sector * sector;
+    const int unit = pitch_align > x1_align ? pitch_align / elem_bytes : sector;
+    g.P = (need + unit - 1) / unit * unit;
     g.PY = g.P * (ny + 2);
     const long long slot_align = 256 / elem_bytes;
     g.S = (g.PY * (nz + 2) + slot_align - 1) / slot_align * slot_align;
@@ -115,6 +116,10 @@ inline Grid make_grid(int nx, int ny, int nz, int elem_bytes, int x1_align = 32)
 
 // Alignment of x = 1 in the rows of batch and server boxes (see above).
 constexpr int kPackedX1Align = 8;
+// Rows of an FP32 batch: whole multiples of the 16 bytes that a tensor copy
+// (lbm_pair.cuh) needs of its strides.  With 32, 64 and 128 bytes the pair kernel took
+// 2-5 %, 6-23 % and 10-36 % longer.  The other storages' batches run without it.
+inline int batch_pitch_align(int storage) { return storage == 1 ? 16 : 0; }
 
 // True for the default layout (x = 1 on a 32-byte boundary).
 inline bool default_layout(const Grid& g, int elem_bytes) { return g.xoff == 32 / elem_bytes - 1; }

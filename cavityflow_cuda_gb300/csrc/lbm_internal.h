@@ -61,6 +61,7 @@ struct lbm_solver {
     int64_t device_bytes = 0;
     bool owns_dd = true;            // false: populations live in a batch's pool
     lbm_batch* batch = nullptr;     // the batch this solver is a domain view of
+    int* batch_err = nullptr;       // the batch's kernel error flag, instead of the solver's
 };
 
 namespace lbm_detail {
@@ -75,10 +76,12 @@ int default_variant(int storage, long long cells);
 int default_batch_variant(int storage);
 // Creates a solver; with `external_dd` its populations live there (a batch
 // pool) and are initialised but never freed by the solver.
-// x1_align: 32 (the default layout) or 8 (the packed rows of batch pools,
-// see make_grid).
-int create_solver(const lbm_params* prm, void* external_dd, lbm_solver** out, int x1_align = 32);
+// x1_align, pitch_align: 32, 0 (the default layout) or those of batch pools'
+// packed rows (see make_grid).
+int create_solver(const lbm_params* prm, void* external_dd, lbm_solver** out, int x1_align = 32, int pitch_align = 0);
 void destroy_solver(lbm_solver* s);
+// Gives back the second pool of a batch; whether there was one.
+bool drop_batch_pairs(lbm_batch* b);
 int* err_flag(lbm_solver* s);
 // Two device words of the solver: [0] the first step of a graph replay,
 // [1] always zero (the base of directly launched steps).

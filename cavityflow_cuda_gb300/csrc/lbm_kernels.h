@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "lbm_core.cuh"
 
 namespace lbm {
@@ -129,6 +131,23 @@ cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid&
 // Whether that kernel can run on this domain and takes less time than the
 // default alpha and beta kernels.
 bool pair_step_pays(int storage, const Grid& g);
+
+// The same for the domains of a batch.  A plan is made once for a batch; its
+// image goes to device memory when a second pool is there.
+struct BatchDomain;
+struct PairBatchPlan {
+    int items = 0;                     // 0: does not pay, or cannot run
+    size_t maps[2] = {0, 0};           // places in the image: copies from the pool, from the second one,
+    size_t domains = 0, domain_of = 0; // the domains, the domain of each item
+    std::vector<unsigned char> image;
+};
+void plan_pair_batch(int storage, const BatchDomain* doms, int count, PairBatchPlan& plan);
+// Fills in the copies' descriptors; false if the driver refuses one.
+bool bind_pair_batch(int storage, const void* pool, const void* pool2, PairBatchPlan& plan);
+// `image`: the plan's image on the device.  `back`: from the second pool to the
+// pool (`out`), else from the pool to the second one (`out`).
+cudaError_t launch_pair_batch(int storage, const PairBatchPlan& plan, const void* image, bool back, void* out,
+                              const uint32_t* step_base, uint32_t step_off, int* work, int* err, cudaStream_t st);
 // Whether a variant fits this domain: its vectors' alignment in the domain's
 // row layout (register variants), shared memory (bulk-copy variants).
 bool fast_variant_fits(int storage, int variant, const Grid& g);
@@ -137,7 +156,6 @@ bool fast_variant_fits(int storage, int variant, const Grid& g);
 void fast_variant_shape(int storage, int variant, bool alpha, int nx, int& cells_per_thread, int& block_threads);
 
 // Batches of box cavities (lbm_fast.cuh): register variants only.
-struct BatchDomain;
 struct BatchArgs {
     void* pool;               // the domains' populations
     const BatchDomain* doms;  // packed table

@@ -2,6 +2,12 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
+#include <cstring>
+#include <functional>
+#include <queue>
+#include <vector>
+
 #include "lbm_kernels.h"
 #include "lbm_pair.cuh"
 
@@ -79,37 +85,230 @@ Split split(const Grid& g, int elem, int sms)
     return s;
 }
 
+// The map of a domain's populations for boxes of `slots` slots, `rows` rows of
+// `row` elements.
 template <class St>
-cudaError_t launch(const void* in, void* out, const Grid& g, const Params& p, int lid_y, int* work, int* err,
-                   cudaStream_t st)
+bool make_map(CUtensorMap& map, const void* in, const Grid& g, int row, int rows, int slots)
 {
-    using bits = typename St::bits;
-    constexpr int TY = Shape<St>::TY, NST = Shape<St>::NST;
-    using S = PairShape<St, kTX, TY, NST>;
     const auto encode = encode_fn();
-    const int sms = sm_count();
-    if (!encode || sms < 1) return cudaErrorNotSupported;
-    constexpr cuuint64_t eb = sizeof(bits);
+    if (!encode) return false;
+    constexpr cuuint64_t eb = sizeof(typename St::bits);
     const cuuint64_t dims[4] = {(cuuint64_t)g.P, (cuuint64_t)g.ny + 2, (cuuint64_t)g.nz + 2, (cuuint64_t)Q};
     const cuuint64_t strides[3] = {(cuuint64_t)g.P * eb, (cuuint64_t)g.PY * eb, (cuuint64_t)g.S * eb};
-    const cuuint32_t box[4] = {(cuuint32_t)S::W, TY + 2, 1, (cuuint32_t)Q}, unit[4] = {1, 1, 1, 1};
-    CUtensorMap map;
-    if (encode(&map, eb == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 4,
-               const_cast<void*>(in), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
-    auto kern = pair_step<St, kTX, TY, NST>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    const cuuint32_t box[4] = {(cuuint32_t)row, (cuuint32_t)rows, 1, (cuuint32_t)slots}, unit[4] = {1, 1, 1, 1};
+    return encode(&map, eb == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 4,
+                  const_cast<void*>(in), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <class St, bool BATCH>
+cudaError_t launch(const CUtensorMap& map, const PairCtx& one, const PairWork& w, const uint32_t* step_base,
+                   uint32_t step_off, int sms, int* err, cudaStream_t st)
+{
+    constexpr int TY = Shape<St>::TY, NST = Shape<St>::NST;
+    using S = PairShape<St, kTX, TY, NST, BATCH>;
+    auto kern = pair_step<St, kTX, TY, NST, BATCH>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
     if (e != cudaSuccess) return e;
-    const Split s = split(g, (int)eb, sms);
-    const PairWork w{(int)s.tiles_x, (int)s.tiles, (int)s.items, s.zc, work};
-    const int grid = s.items < sms ? (int)s.items : sms;
-    return launch_step(kern, dim3((unsigned)grid), S::THREADS, st, S::SMEM, map, pair_slots(out, g, (int)eb), g,
-                       (float)p.inv_tau, (float)p.lid_u, lid_y, p.wall_y, p.step_base, p.step_off, w, err);
+    const int grid = w.items < sms ? w.items : sms;
+    return launch_step(kern, dim3((unsigned)grid), S::THREADS, st, S::SMEM, map, one, step_base, step_off, w, err);
+}
+
+template <class St>
+cudaError_t launch_one(const void* in, void* out, const Grid& g, const Params& p, int lid_y, int* work, int* err,
+                       cudaStream_t st)
+{
+    constexpr int TY = Shape<St>::TY, eb = (int)sizeof(typename St::bits);
+    const int sms = sm_count();
+    CUtensorMap map;
+    if (sms < 1 || !make_map<St>(map, in, g, pair_row<St>(kTX), TY + 2, Q)) return cudaErrorNotSupported;
+    const Split s = split(g, eb, sms);
+    const PairCtx one{g, pair_slots(out, g, eb), {kTX, TY, pair_row<St>(kTX)}, (int)s.tiles_x, (int)s.tiles, s.zc, 0,
+                      (float)p.inv_tau, (float)p.lid_u, lid_y, p.wall_y};
+    const PairWork w{(int)s.items, work, nullptr, nullptr, nullptr, nullptr};
+    return launch<St, false>(map, one, w, p.step_base, p.step_off, sms, err, st);
+}
+
+// Microseconds of a plane of a block with full tiles of 64 cells, GB300.
+constexpr double kPlane[5] = {0, 1.80, 1.70, 1.67, 1.96};
+
+// Tiles for a domain of a batch (FP32): the shape whose planes of the whole
+// domain take the least time.  A plane's time, fitted to 45 shapes from 12 x 32
+// to 128 x 3 (7 % off on average): its cells', and its rows', which a warp's
+// accesses straddle and the copies bring one by one.  Microseconds, GB300: 64 x 8
+// 2.5-2.8, 96 x 5 2.65, 48 x 10 2.5-2.7, 32 x 16 3.1-3.4, 14 x 32 3.8.
+template <class St>
+PairDims batch_dims(const Grid& g, double& plane)
+{
+    constexpr int TY = Shape<St>::TY, NST = Shape<St>::NST;
+    PairDims best{0, 0, 0};
+    double best_cost = 0;
+    for (int nt = 1, last = 0; nt <= g.nx; ++nt) {
+        const int tx = ((g.nx + nt - 1) / nt + 1) / 2 * 2;
+        if (tx < 8 && nt > 1) break;
+        if (tx == last || tx > (nt == 1 ? 96 : kTX)) continue;  // wider ones leave room for few rows
+        last = tx;
+        int ty = 0;
+        while (pair_dims_fit<St, kTX, TY, NST>(tx, ty + 1)) ++ty;
+        if (ty == 0) continue;
+        const int rows = (g.ny + ty - 1) / ty;
+        ty = (g.ny + rows - 1) / rows;
+        const double cost = std::max(2.3, 0.0046 * tx * ty + 0.0546 * (ty + 2));
+        const double total = cost * rows * ((g.nx + tx - 1) / tx);
+        if (best.tx == 0 || total < best_cost) {
+            best = {tx, ty, pair_row<St>(tx)};
+            best_cost = total;
+            plane = cost;
+        }
+    }
+    return best;
+}
+
+template <class St>
+void plan_batch(int storage, const BatchDomain* doms, int count, PairBatchPlan& plan)
+{
+    constexpr int eb = (int)sizeof(typename St::bits);
+    const int sms = sm_count();
+    if (sms < 1 || !encode_fn()) return;
+    std::vector<PairDomain> table((size_t)count);
+    std::vector<double> plane((size_t)count);
+    double cells = 0, state = 0;
+    for (int i = 0; i < count; ++i) {
+        const BatchDomain& b = doms[i];
+        PairDomain& d = table[(size_t)i];
+        if (b.g.P * eb % 16 != 0 || (unsigned long long)b.g.S * eb >= (1ull << 32) || b.step0 != 0) return;
+        d.g = b.g;
+        d.offset = b.offset;
+        d.dims = batch_dims<St>(b.g, plane[(size_t)i]);
+        if (d.dims.tx == 0) return;
+        d.tiles_x = (b.g.nx + d.dims.tx - 1) / d.dims.tx;
+        d.tiles = d.tiles_x * ((b.g.ny + d.dims.ty - 1) / d.dims.ty);
+        d.inv_tau = (float)b.inv_tau;
+        d.lid_u = (float)b.lid_u;
+        d.lid_y = b.lid_y;
+        d.wall_y = b.wall_y;
+        cells += (double)b.g.nx * b.g.ny * b.g.nz;
+        state += (double)Q * (double)b.g.S * eb;
+    }
+    // Chunks: long ones repeat fewer planes, short ones fill the chip and its last
+    // turns.  The longest items come first, so that the last ones to run are short.
+    auto chunk = [&](const PairDomain& d, int zmax) {
+        const int n = (d.g.nz + zmax - 1) / zmax;
+        return (d.g.nz + n - 1) / n;
+    };
+    auto count_of = [&](const PairDomain& d, int zc) { return (long long)d.tiles * ((d.g.nz + zc - 1) / zc); };
+    std::vector<int> order((size_t)count), best_order;
+    std::vector<double> cost((size_t)count);
+    double best = 0;
+    int best_z = 0;
+    for (const int zmax : {32, 24, 16, 12, 8}) {
+        long long items = 0;
+        double total = 0;
+        for (int i = 0; i < count; ++i) {
+            const PairDomain& d = table[(size_t)i];
+            const int zc = chunk(d, zmax);
+            order[(size_t)i] = i;
+            cost[(size_t)i] = plane[(size_t)i] * (zc + 2) + 2.0;
+            items += count_of(d, zc);
+            total += (double)count_of(d, zc) * cost[(size_t)i];
+        }
+        if (items > (1 << 24)) return;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[(size_t)a] > cost[(size_t)b]; });
+        double time = total / sms;
+        if (items <= 64 * sms) {  // otherwise the last turn does not matter
+            std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+            for (int i = 0; i < sms; ++i) free_at.push(0);
+            time = 0;
+            for (const int i : order)
+                for (long long n = count_of(table[(size_t)i], chunk(table[(size_t)i], zmax)); n > 0; --n) {
+                    const double end = free_at.top() + cost[(size_t)i];
+                    free_at.pop();
+                    free_at.push(end);
+                    time = std::max(time, end);
+                }
+        }
+        if (best_z == 0 || time < best) {
+            best = time;
+            best_z = zmax;
+            best_order = order;
+        }
+    }
+    // Measured: 0.86-1.0 of `best` for 26 batches from 8 cavities of 8 .. 96 cells an edge to 610 of 32^3, where the
+    // batch kernels step 34-38 cells a nanosecond from memory and 45 from L2.
+    if (4.0 + 0.95 * best >= 0.98 * 2.0 * cells / (state < 100e6 ? 45000 : 36000)) return;
+    int items = 0;
+    std::vector<int> domain_of;
+    for (const int i : best_order) {
+        PairDomain& d = table[(size_t)i];
+        d.zc = chunk(d, best_z);
+        d.item0 = items;
+        const int n = (int)count_of(d, d.zc);
+        items += n;
+        domain_of.insert(domain_of.end(), (size_t)n, i);
+    }
+    plan.maps[0] = 0;
+    plan.maps[1] = (size_t)count * sizeof(CUtensorMap);
+    plan.domains = 2 * plan.maps[1];
+    plan.domain_of = plan.domains + table.size() * sizeof(PairDomain);
+    plan.image.resize(plan.domain_of + domain_of.size() * sizeof(int));
+    std::memcpy(plan.image.data() + plan.domains, table.data(), table.size() * sizeof(PairDomain));
+    std::memcpy(plan.image.data() + plan.domain_of, domain_of.data(), domain_of.size() * sizeof(int));
+    plan.items = items;
+}
+
+template <class St>
+bool bind_batch(const void* pool, const void* pool2, PairBatchPlan& plan)
+{
+    const size_t count = plan.maps[1] / sizeof(CUtensorMap);
+    for (size_t i = 0; i < count; ++i) {
+        PairDomain d;
+        std::memcpy(&d, plan.image.data() + plan.domains + i * sizeof(d), sizeof(d));
+        for (int k = 0; k < 2; ++k) {
+            CUtensorMap map;
+            const char* base = static_cast<const char*>(k ? pool2 : pool) + d.offset * (long long)sizeof(typename St::bits);
+            if (!make_map<St>(map, base, d.g, d.dims.w, d.dims.ty + 2, 1)) return false;
+            std::memcpy(plan.image.data() + plan.maps[k] + i * sizeof(map), &map, sizeof(map));
+        }
+    }
+    return true;
+}
+
+template <class St>
+cudaError_t launch_batch(const PairBatchPlan& plan, const void* image, bool back, void* out, const uint32_t* step_base,
+                         uint32_t step_off, int* work, int* err, cudaStream_t st)
+{
+    const int sms = sm_count();
+    if (sms < 1) return cudaErrorNotSupported;
+    const char* const at = static_cast<const char*>(image);
+    const PairWork w{plan.items, work, reinterpret_cast<const PairDomain*>(at + plan.domains),
+                     reinterpret_cast<const int*>(at + plan.domain_of),
+                     reinterpret_cast<const CUtensorMap*>(at + plan.maps[back ? 1 : 0]), out};
+    const CUtensorMap no_map{};
+    const PairCtx no_domain{};
+    return launch<St, true>(no_map, no_domain, w, step_base, step_off, sms, err, st);
 }
 
 }  // namespace
+
+void plan_pair_batch(int storage, const BatchDomain* doms, int count, PairBatchPlan& plan)
+{
+    plan = PairBatchPlan{};
+    if (storage == 1) plan_batch<F32>(storage, doms, count, plan);
+}
+
+bool bind_pair_batch(int storage, const void* pool, const void* pool2, PairBatchPlan& plan)
+{
+    return storage == 1 && bind_batch<F32>(pool, pool2, plan);
+}
+
+cudaError_t launch_pair_batch(int storage, const PairBatchPlan& plan, const void* image, bool back, void* out,
+                              const uint32_t* step_base, uint32_t step_off, int* work, int* err, cudaStream_t st)
+{
+    if (storage != 1) return cudaErrorInvalidValue;
+    add_launches(1);
+    return launch_batch<F32>(plan, image, back, out, step_base, step_off, work, err, st);
+}
 
 bool pair_step_pays(int storage, const Grid& g)
 {
@@ -124,13 +323,12 @@ bool pair_step_pays(int storage, const Grid& g)
     // Measured on GB300, microseconds: a plane of a block, and the separate
     // kernels' cells per microsecond from memory and, while the state fits L2,
     // from there (the pair kernel works on two arrays and so never does).
-    static const double plane[5] = {0, 1.80, 1.70, 1.67, 1.96};
     static const double rate[5] = {0, 43000, 80000, 80000, 79000};
     static const double rate_l2[5] = {0, 54000, 75000, 75000, 70000};
     const double state = (double)Q * (double)g.S * eb;
     const double cells = (double)g.nx * g.ny * g.nz;
     const double separate = 2.0 * cells / (state < 100e6 ? rate_l2 : rate)[storage];
-    return 6.0 + (double)s.planes * plane[storage] < 0.97 * separate;
+    return 6.0 + (double)s.planes * kPlane[storage] < 0.97 * separate;
 }
 
 cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid& g, const Params& p, int lid_y,
@@ -138,10 +336,10 @@ cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid&
 {
     add_launches(1);
     switch (storage) {
-    case 1: return launch<F32>(in, out, g, p, lid_y, work, err, st);
-    case 2: return launch<F16S>(in, out, g, p, lid_y, work, err, st);
-    case 3: return launch<BF16S>(in, out, g, p, lid_y, work, err, st);
-    case 4: return launch<F16SR>(in, out, g, p, lid_y, work, err, st);
+    case 1: return launch_one<F32>(in, out, g, p, lid_y, work, err, st);
+    case 2: return launch_one<F16S>(in, out, g, p, lid_y, work, err, st);
+    case 3: return launch_one<BF16S>(in, out, g, p, lid_y, work, err, st);
+    case 4: return launch_one<F16SR>(in, out, g, p, lid_y, work, err, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -9,7 +9,7 @@
 //
 // A block owns a tile of TX x TY cells and marches along z.  Per plane:
 //   1. a warp has TMA bring the 19 slots of the tile and of a one-cell frame
-//      around it into a shared-memory stage (one box a plane);
+//      around it into a shared-memory stage (one box a plane; for batches a box a slot);
 //   2. the alpha threads collide tile and frame in place: population k of a
 //      cell goes to slot opp(k) of that cell, wall cells stay as they are,
 //      exactly as alpha leaves the array (the frame's cells are collided again
@@ -37,6 +37,16 @@
 // 1.41 -> 1.28 (88.8 GLUP/s; its dither is a fifth of its instructions).  The
 // 16-bit storages are bound by issue slots and the FP32 pipe (54-60 % of the
 // slots used), not by memory.
+//
+// Batches (FP32): the items of all domains in one launch, the longest first, with
+// the tiles of each domain as they fit it best (batch_dims in lbm_pair.cu) and a
+// domain's layout and parameters in shared memory.  Same kernel, BATCH: a full
+// tile's plane takes 2.1 us instead of 1.9, 0.1 of it for 19 copies in place of
+// one and for addresses from shared memory, the rest for rows that start 8 bytes
+// past a sector.  GLUP/s, the separate kernels -> this one: 64 and 512 cavities
+// of 16 .. 96 cells an edge 35.8 -> 43.8 and 34.4 -> 45.0, 76 of 64^3 37 -> 52,
+// 610 of 32^3 34.7 -> 42.  The 16-bit storages stay with the separate kernels:
+// they move half the bytes and ran at 0.75 .. 1.0 of their speed here.
 #pragma once
 
 #include <cstdint>
@@ -243,11 +253,11 @@ struct Two<St, true> {
         f2_split(F2{r}, a, b);
         return b;
     }
-    // the cells at p[DX] and p[DX + SEP]
-    template <int DX, int SEP>
-    __device__ static raw load_at(const float* p)
+    // the cells at p[DX] and p[DX + sep]
+    template <int DX>
+    __device__ static raw load_at(const float* p, int sep)
     {
-        return join(p[DX], p[DX + SEP]);
+        return join(p[DX], p[DX + sep]);
     }
     __device__ static F2 widen(raw r) { return F2{r}; }
     __device__ static raw narrow(F2 v, uint32_t, uint32_t, int) { return v.v; }
@@ -262,9 +272,9 @@ struct Two<St, false> {
     __device__ static raw join(bits a, bits b) { return (raw)a | ((raw)b << 16); }
     __device__ static bits first(raw r) { return (bits)(r & 0xffffu); }
     __device__ static bits second(raw r) { return (bits)(r >> 16); }
-    // the cells at p[DX] and p[DX + 1], p aligned to a word (SEP is 1)
-    template <int DX, int SEP>
-    __device__ static raw load_at(const bits* p)
+    // the cells at p[DX] and p[DX + 1], p aligned to a word (sep is 1)
+    template <int DX>
+    __device__ static raw load_at(const bits* p, int)
     {
         if constexpr (DX == 0) return load(p);
         else if constexpr (DX == 1) return __byte_perm(load(p), load(p + 2), 0x5432);
@@ -279,30 +289,46 @@ struct Two<St, false> {
     }
 };
 
-// Geometry of one shape: TX x TY cells, NST stages.  A stage is a box of the
-// population array: all 19 slots, the tile's rows and one on either side, and
-// from 16 bytes left of the tile's first cell to 16 bytes right of its last
-// (TMA copies start and end on 16-byte boundaries).
-template <class St, int TX, int TY, int NST>
+// Tiles.  A stage holds, of one plane, all 19 slots (SLOT elements apart) of the
+// tile's rows and one on either side, from a 16-byte boundary left of the tile's
+// left neighbour column to one right of its right neighbour column (TMA copies
+// start and end on such boundaries).  The threads are those of TX x TY cells;
+// other shapes that need no more of them, and no more room, run on the kernel of
+// batches (PairDims), so that the tiles fit each cavity.
+template <class St, int TX, int TY, int NST, bool BATCH>
 struct PairShape {
     using bits = typename St::bits;
-    static constexpr int LX = 16 / (int)sizeof(bits);            // column of the tile's first cell
-    static constexpr int W = TX + 2 * LX;                        // stage row
-    static constexpr int SLOT = (TY + 2) * W;                    // stage slot
-    static constexpr int STAGE = (Q * SLOT * (int)sizeof(bits) + 127) / 128 * 128 / (int)sizeof(bits);
-    static constexpr uint32_t BYTES = (uint32_t)(Q * SLOT * sizeof(bits));
-    static constexpr int PAIRS = (TY + 2) * (TX / 2);              // pairs of cells of tile rows -1 .. TY
-    static constexpr int NA = (PAIRS + 2 * (TY + 2) + 31) / 32 * 32;  // alpha threads: also the frame's columns
-    static constexpr int NB = TY * (TX / 2);                       // beta threads
+    static constexpr int kAlign = 16 / (int)sizeof(bits);        // elements to a 16-byte boundary
+    static constexpr int kUnit = 128 / (int)sizeof(bits);        // of a copy's destination
+    static constexpr int kSlot = (TY + 2) * (TX + 2 * kAlign);
+    static constexpr int SLOT = BATCH ? (kSlot + kUnit - 1) / kUnit * kUnit : kSlot;
+    static constexpr int STAGE = (Q * SLOT + kUnit - 1) / kUnit * kUnit;
+    static constexpr int NA = ((TY + 2) * (TX / 2 + 2) + 31) / 32 * 32;  // alpha threads: pairs of tile rows -1 .. TY, the frame's columns
+    static constexpr int NB = TY * (TX / 2);                     // beta threads
     static constexpr int THREADS = NA + NB + 32;                 // and the warp that issues the copies
     static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(bits) + NST * (sizeof(uint64_t) + sizeof(int));
-    // the two cells of a beta thread: FP32 half a row apart, so that each access
-    // of a warp is one run of 4-byte elements whatever the shift; 16-bit neighbours,
-    // one word
-    static constexpr int SEP = sizeof(bits) == 4 ? TX / 2 : 1;
     static_assert(NB % 32 == 0, "whole warps");
     static_assert(1 + 2 * NST <= 15, "named barriers");
 };
+
+// A tile's cells along x (even) and y, and the elements of a stage row.
+struct PairDims {
+    int tx, ty, w;
+};
+template <class St>
+__host__ __device__ constexpr int pair_row(int tx)
+{
+    const int align = 16 / (int)sizeof(typename St::bits);
+    // the tile's first cell is at most `align` columns in, and one follows its last
+    return tx % align == 0 ? tx + 2 * align : (align + tx + 1 + align - 1) / align * align;
+}
+template <class St, int TX, int TY, int NST>
+constexpr bool pair_dims_fit(int tx, int ty)
+{
+    using S = PairShape<St, TX, TY, NST, true>;
+    return tx >= 2 && tx % 2 == 0 && ty >= 1 && (ty + 2) * (tx / 2 + 2) <= S::NA && ty * (tx / 2) <= S::NB &&
+           (ty + 2) * pair_row<St>(tx) <= S::SLOT && pair_row<St>(tx) <= 256 && ty + 2 <= 256;
+}
 
 // Named barriers, as a producer and a consumer use them: `arrive` does not wait.
 __device__ __forceinline__ void named_sync(int id, int threads)
@@ -314,26 +340,102 @@ __device__ __forceinline__ void named_arrive(int id, int threads)
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// The work of one launch: the tiles of every z chunk, chunks slowest.  Blocks
-// are persistent and take the next item from a counter, so that at any time
-// they work on neighbouring tiles of the same planes and find each other's
-// frames in L2; a block's copies run ahead into its next item.
+// Where the slots of `out` are: own[k] + o is slot k of the cell at byte o of
+// its slot, push[k] + o the place in slot k, one plane below, that the cell
+// pushes population k to.  Uniform bases and a 32-bit offset a thread: one
+// address per access instead of a 64-bit sum.
+struct PairSlots {
+    char* own[Q];
+    char* push[Q];
+};
+inline PairSlots pair_slots(void* out, const Grid& g, int elem)
+{
+    PairSlots s;
+    for (int k = 0; k < Q; ++k) {
+        s.own[k] = static_cast<char*>(out) + (long long)k * g.S * elem;
+        s.push[k] = s.own[k] + ((dir_z(k) - 1) * g.PY + dir_y(k) * g.P + dir_x(k)) * elem;
+    }
+    return s;
+}
+
+// A domain as the threads of the kernel see it.
+struct PairCtx {
+    Grid g;
+    PairSlots slots;
+    PairDims dims;       // of its tiles
+    int tiles_x, tiles;  // tiles of a row, of a plane
+    int zc;              // planes of a chunk
+    int item;            // batches: the item in work, counted within the domain
+    float inv_tau, lid_u;
+    int lid_y, wall_y;
+};
+
+// A domain of a batch: PairCtx is made of it when one of its items comes up.
+struct PairDomain {
+    Grid g;
+    long long offset;  // elements from the pool's base
+    PairDims dims;
+    int tiles_x, tiles, zc;
+    int item0;         // its first item
+    float inv_tau, lid_u;
+    int lid_y, wall_y;
+};
+
+// The work of one launch: items, each a tile of a z chunk (of a domain), chunks
+// slowest.  Blocks are persistent and take the next item from a counter, so
+// that at any time they work on neighbouring tiles of the same planes and find
+// each other's frames in L2; a block's copies run ahead into its next item.
 struct PairWork {
-    int tiles_x, tiles, items;  // tiles of a row, of a plane; items in all
-    int zc;                     // planes of a chunk
+    int items;
     int* next;                  // [0] items taken beyond the first of each block, [1] blocks done; zero between launches
+    const PairDomain* domains;  // batches: the domains, the domain of each item, the copies' maps of each
+    const int* domain_of;       // domain's array, the array written to
+    const CUtensorMap* maps;
+    void* out;
 };
 struct PairItem {
     int x0, y0, za, zb;  // first cell, first and last plane
 };
-template <int TX, int TY>
-__device__ __forceinline__ PairItem pair_item(const PairWork& w, const Grid& g, int item)
+__device__ __forceinline__ PairItem pair_item(const PairCtx& c, const PairDims& d, int item)
 {
-    const int chunk = item / w.tiles, t = item - chunk * w.tiles;
-    const int ty = t / w.tiles_x, tx = t - ty * w.tiles_x;
-    const int za = 1 + chunk * w.zc;
-    return {1 + tx * TX, 1 + ty * TY, za, min(g.nz, za + w.zc - 1)};
+    const int chunk = item / c.tiles, t = item - chunk * c.tiles;
+    const int ty = t / c.tiles_x, tx = t - ty * c.tiles_x;
+    const int za = 1 + chunk * c.zc;
+    return {1 + tx * d.tx, 1 + ty * d.ty, za, min(c.g.nz, za + c.zc - 1)};
 }
+// First column of a stage row: the last 16-byte boundary left of the tile's left
+// neighbour column.
+template <class St>
+__device__ __forceinline__ int pair_column(const Grid& g, int x0)
+{
+    return (g.xoff + x0 - 1) & ~(16 / (int)sizeof(typename St::bits) - 1);
+}
+
+// Where the threads find the domain of an item.  One domain: the kernel's
+// parameters, tiles of TX x TY.  A batch: shared memory, where the copying warp
+// puts it; a block has at most three items between its stages and that warp.
+constexpr int kPairContexts = 4;
+template <class St, int TX, int TY, bool BATCH>
+struct PairSource {
+    const PairCtx& one;
+    PairCtx* many;
+    __device__ __forceinline__ const PairCtx& at(int item) const
+    {
+        if constexpr (BATCH) return many[item & (kPairContexts - 1)];
+        else return one;
+    }
+    __device__ __forceinline__ PairDims dims(int item) const
+    {
+        if constexpr (BATCH) return at(item).dims;
+        else return {TX, TY, pair_row<St>(TX)};
+    }
+    __device__ __forceinline__ PairItem item(int n) const
+    {
+        if constexpr (BATCH) return pair_item(at(n), dims(n), at(n).item);
+        else return pair_item(one, dims(n), n);
+    }
+};
+
 // Waits until the phase with `parity` of `bar` has completed, at most limit_ns
 // (tma::mbar_wait with the hardware's own wait between the looks).
 __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns)
@@ -355,24 +457,6 @@ __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, uint64
     }
 }
 
-// Where the slots of `out` are: own[k] + o is slot k of the cell at byte o of
-// its slot, push[k] + o the place in slot k, one plane below, that the cell
-// pushes population k to.  Uniform bases and a 32-bit offset a thread: one
-// address per access instead of a 64-bit sum.
-struct PairSlots {
-    char* own[Q];
-    char* push[Q];
-};
-inline PairSlots pair_slots(void* out, const Grid& g, int elem)
-{
-    PairSlots s;
-    for (int k = 0; k < Q; ++k) {
-        s.own[k] = static_cast<char*>(out) + (long long)k * g.S * elem;
-        s.push[k] = s.own[k] + ((dir_z(k) - 1) * g.PY + dir_y(k) * g.P + dir_x(k)) * elem;
-    }
-    return s;
-}
-
 // The slots that point away from the low (SIGN 1) or high (-1) wall of an axis.
 template <int AXIS, int SIGN>
 struct FromFace {
@@ -388,21 +472,56 @@ __host__ __device__ constexpr int z_rank(int k)
 }
 
 // The copying warp: takes items and brings the planes za - 1 .. zb + 1 of each
-// into the stages, as beta gives them back.  item_of[s] tells the others what
-// stage s holds; -1 ends the block.
-template <class St, int TX, int TY, int NST>
-__device__ __forceinline__ void pair_copy(const CUtensorMap* map, const Grid& g, const PairWork& w,
-                                          typename St::bits* smem, uint64_t* full, int* item_of)
+// into the stages, as beta gives them back.  item_of[s] tells the others which
+// item stage s holds (one domain: its number; a batch: the block's how-manieth);
+// -1 ends the block.
+template <class St, int TX, int TY, int NST, bool BATCH>
+__device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSource<St, TX, TY, BATCH>& src,
+                                          const PairWork& w, typename St::bits* smem, uint64_t* full, int* item_of)
 {
-    using S = PairShape<St, TX, TY, NST>;
-    const bool lead = (threadIdx.x & 31) == 0;
-    int stage = 0, used = 0, item = (int)blockIdx.x;
+    using S = PairShape<St, TX, TY, NST, BATCH>;
+    using bits = typename St::bits;
+    const int lane = (int)threadIdx.x & 31;
+    const bool lead = lane == 0;
+    int stage = 0, used = 0, item = (int)blockIdx.x, seen = 0;
     // `in`, `out` and the counters are the previous step's until it is complete; the other threads touch global memory
     // only after this warp's first copy has arrived
     wait_previous_step();
 #pragma unroll 1
     while (item < w.items) {
-        const PairItem it = pair_item<TX, TY>(w, g, item);
+        const int n = BATCH ? seen++ : item;
+        if constexpr (BATCH) {
+            const int dom = w.domain_of[item];
+            const PairDomain& d = w.domains[dom];
+            PairCtx& c = src.many[n & (kPairContexts - 1)];
+            const Grid g = d.g;
+            static_for<0, Q>([&](auto kc) {
+                constexpr int k = decltype(kc)::value;
+                if (lane == k) {
+                    char* const own = static_cast<char*>(w.out) + (d.offset + k * g.S) * (long long)sizeof(bits);
+                    c.slots.own[k] = own;
+                    c.slots.push[k] = own + ((dir_z(k) - 1) * g.PY + dir_y(k) * g.P + dir_x(k)) * (long long)sizeof(bits);
+                }
+            });
+            if (lane == Q) {
+                c.g = g;
+                c.dims = d.dims;
+                c.tiles_x = d.tiles_x;
+                c.tiles = d.tiles;
+                c.zc = d.zc;
+                c.item = item - d.item0;
+                c.inv_tau = d.inv_tau;
+                c.lid_u = d.lid_u;
+                c.lid_y = d.lid_y;
+                c.wall_y = d.wall_y;
+            }
+            __syncwarp();
+            map = w.maps + dom;
+            if (lead) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+        }
+        const PairItem it = src.item(n);
+        const PairDims dims = src.dims(n);
+        const int col = pair_column<St>(src.at(n).g, it.x0);
         int next = 0;
 #pragma unroll 1
         for (int p = it.za - 1; p <= it.zb + 1; ++p) {
@@ -410,15 +529,18 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const Grid& g,
             if (used == NST) named_sync(1 + NST + stage, S::NB + 32);
             else ++used;
             if (lead) {
-                item_of[stage] = item;
+                item_of[stage] = n;
                 tma::fence_proxy_async();  // alpha's and beta's accesses to the stage, before the copy overwrites it
-                tma::mbar_arrive_expect_tx(&full[stage], S::BYTES);
-                asm volatile(
-                    "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-                    "%5}], [%6];" ::"r"(tma::smem_addr(smem + stage * S::STAGE)),
-                    "l"(map), "r"(g.xoff + it.x0 - S::LX), "r"(it.y0 - 1), "r"(p), "r"(0),
-                    "r"(tma::smem_addr(&full[stage]))
-                    : "memory");
+                tma::mbar_arrive_expect_tx(&full[stage], (uint32_t)(Q * (dims.ty + 2) * dims.w * (int)sizeof(bits)));
+                const uint32_t to = tma::smem_addr(smem + stage * S::STAGE), bar = tma::smem_addr(&full[stage]);
+                // all slots in one box; a batch's boxes are of many sizes, the slots' places in a stage are not
+#pragma unroll 1
+                for (int k = 0; k < (BATCH ? Q : 1); ++k)
+                    asm volatile(
+                        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+                        "%4, %5}], [%6];" ::"r"(to + (uint32_t)(k * S::SLOT * (int)sizeof(bits))),
+                        "l"(map), "r"(col), "r"(it.y0 - 1), "r"(p), "r"(k), "r"(bar)
+                        : "memory");
             }
             stage = stage + 1 == NST ? 0 : stage + 1;
         }
@@ -441,24 +563,16 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const Grid& g,
 }
 
 // Alpha threads: collide the cells of a stage in place.
-template <class St, int TX, int TY, int NST>
-__device__ __forceinline__ void pair_alpha(const Grid& g, const float inv_tau, const float lid_u, const int lid_y,
-                                           const int wall_y, const PairWork& w, const uint32_t step,
+template <class St, int TX, int TY, int NST, bool BATCH>
+__device__ __forceinline__ void pair_alpha(const PairSource<St, TX, TY, BATCH>& src, const uint32_t step,
                                            typename St::bits* __restrict__ smem, uint64_t* full,
                                            const int* item_of, int* __restrict__ err)
 {
-    using S = PairShape<St, TX, TY, NST>;
+    using S = PairShape<St, TX, TY, NST, BATCH>;
     using bits = typename St::bits;
     using two = Two<St>;
-    // Pairs of tile rows -1 .. TY, then two cells left and two right of each of
-    // these rows, of which the frame has the nearer one; the other cell of such
-    // a pair is collided from whatever the stage holds, and nothing reads it.
     const int tid = (int)threadIdx.x;
-    const bool column = tid >= S::PAIRS;
-    const int c = tid - S::PAIRS;
-    const int ry = column ? (c < TY + 2 ? c : c - (TY + 2)) : tid / (TX / 2);
-    const int px = !column ? tid % (TX / 2) : c < TY + 2 ? -1 : TX / 2;
-    bits* const own = smem + ry * S::W + S::LX + 2 * px;
+    bits* own = smem;
     int stage = 0;
     uint32_t phase = 0;
     uint64_t limit_ns = tma::kWaitLimitNs;
@@ -478,28 +592,39 @@ __device__ __forceinline__ void pair_alpha(const Grid& g, const float inv_tau, c
         if (now != item) {  // another tile's first plane
             if (now < 0) break;
             item = now;
-            const PairItem it = pair_item<TX, TY>(w, g, item);
+            const PairItem it = src.item(item);
+            const PairDims d = src.dims(item);
+            const Grid& g = src.at(item).g;
+            // Pairs of tile rows -1 .. ty, then two cells left and two right of each of these rows, of which the frame
+            // has the nearer one; the other cell of such a pair is collided from whatever the stage holds, and nothing
+            // reads it.
+            const int c = tid - (d.ty + 2) * (d.tx / 2);
+            const bool column = c >= 0;
+            const int ry = column ? (c < d.ty + 2 ? c : c - (d.ty + 2)) : tid / (d.tx / 2);
+            const int px = !column ? tid % (d.tx / 2) : c < d.ty + 2 ? -1 : d.tx / 2;
             p = it.za - 1;
             y = it.y0 - 1 + ry;
             xa = it.x0 + 2 * px;
             const int x = column && px < 0 ? xa + 1 : xa;  // the cell that decides
-            work = ry <= TY + 1 && y >= 1 && y <= g.ny && x >= 1 && x <= g.nx;
+            work = ry <= d.ty + 1 && y >= 1 && y <= g.ny && x >= 1 && x <= g.nx;
             both = column || xa < g.nx;
-            lid = y == lid_y;
-            wall = y == wall_y;
+            lid = y == src.at(item).lid_y;
+            wall = y == src.at(item).wall_y;
+            own = smem + ry * d.w + (g.xoff + xa - pair_column<St>(g, it.x0));
         }
+        const PairCtx& ctx = src.at(item);
         bits* const sb = own + stage * S::STAGE;
-        if (p >= 1 && p <= g.nz && work) {
+        if (p >= 1 && p <= ctx.g.nz && work) {
             uint32_t ha = 0, hb = 0;
             if constexpr (St::stochastic) {
-                const uint32_t rh = sr_hash((uint32_t)g.ref(0, y, p), step);
+                const uint32_t rh = sr_hash((uint32_t)ctx.g.ref(0, y, p), step);
                 ha = sr_cell(rh, xa);
                 hb = sr_cell(rh, xa + 1);
             }
             F2 f[Q];
 #pragma unroll
             for (int k = 0; k < Q; ++k) f[k] = two::widen(two::load(sb + k * S::SLOT));
-            cell_rule2<St>(f, lid, wall, inv_tau, lid_u);
+            cell_rule2<St>(f, lid, wall, ctx.inv_tau, ctx.lid_u);
             if (both) {
 #pragma unroll
                 for (int k = 0; k < Q; ++k) two::store(sb + opp(k) * S::SLOT, two::narrow(f[k], ha, hb, k));
@@ -518,25 +643,24 @@ __device__ __forceinline__ void pair_alpha(const Grid& g, const float inv_tau, c
 }
 
 // Beta threads: pull, collide, push to `out`.
-template <class St, int TX, int TY, int NST>
-__device__ __forceinline__ void pair_beta(const PairSlots& slots, const Grid& g, const float inv_tau,
-                                          const float lid_u, const int lid_y, const int wall_y, const PairWork& w,
-                                          const uint32_t step, typename St::bits* __restrict__ smem, const int* item_of)
+template <class St, int TX, int TY, int NST, bool BATCH>
+__device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& src, const uint32_t step,
+                                          typename St::bits* __restrict__ smem, const int* item_of)
 {
-    using S = PairShape<St, TX, TY, NST>;
+    using S = PairShape<St, TX, TY, NST, BATCH>;
     using bits = typename St::bits;
     using two = Two<St>;
     using raw = typename two::raw;
+    constexpr bool k16 = sizeof(bits) == 2;
     const int tid = (int)threadIdx.x - S::NA;
-    const int ry = tid / (TX / 2), px = tid % (TX / 2);
-    constexpr int SEP = S::SEP;
-    const int dx = SEP == 1 ? 2 * px : px;
-    const bits* const own = smem + (ry + 1) * S::W + S::LX + dx;
-    const uint32_t pitch = (uint32_t)(g.PY * (long long)sizeof(bits));
+    const bits* own = smem;
     raw c0[9], m1[5], m2[5];
     int stage = 0, item = -1, p = 0, za = 0, zb = 0, y = 0, xa = 0;
+    // The thread's two cells: FP32 half a row apart, so that each access of a warp is runs of 4-byte elements whatever
+    // the shift; 16-bit neighbours, one word.
+    int SEP = k16 ? 1 : TX / 2, W = pair_row<St>(TX);
     bool tile = false, vb = false, lid = false, wall = false, edge = false;
-    uint32_t off = 0;  // of (xa, y, p) in a slot, bytes
+    uint32_t off = 0, pitch = 0;  // of (xa, y, p) in a slot, of a plane, bytes
 #pragma unroll 1
     for (;;) {
         named_sync(1 + stage, S::NA + S::NB);
@@ -546,19 +670,29 @@ __device__ __forceinline__ void pair_beta(const PairSlots& slots, const Grid& g,
         if (now != item) {  // another tile's first plane
             if (now < 0) break;
             item = now;
-            const PairItem it = pair_item<TX, TY>(w, g, item);
+            const PairItem it = src.item(item);
+            const PairDims d = src.dims(item);
+            const Grid& g = src.at(item).g;
+            const int ry = tid / (d.tx / 2), px = tid % (d.tx / 2);
+            if (BATCH && !k16) SEP = d.tx / 2;
+            if (BATCH) W = d.w;
             za = it.za;
             zb = it.zb;
             p = za - 1;
             y = it.y0 + ry;
-            xa = it.x0 + dx;
-            tile = y <= g.ny && xa <= g.nx;
+            xa = it.x0 + (k16 ? 2 * px : px);
+            tile = ry < d.ty && y <= g.ny && xa <= g.nx;
             vb = xa + SEP <= g.nx;
-            lid = y == lid_y;
-            wall = y == wall_y;
+            lid = y == src.at(item).lid_y;
+            wall = y == src.at(item).wall_y;
             edge = xa == 1 || xa == g.nx || xa + SEP == g.nx || y == 1 || y == g.ny;
             off = (uint32_t)(g.idx(xa, y, p) * (long long)sizeof(bits));
+            pitch = (uint32_t)(g.PY * (long long)sizeof(bits));
+            own = smem + (ry + 1) * d.w + (g.xoff + xa - pair_column<St>(g, it.x0));
         }
+        const PairCtx& ctx = src.at(item);
+        const Grid& g = ctx.g;
+        const PairSlots& slots = ctx.slots;
         if (tile) {
             const bits* const sb = own + stage * S::STAGE;
             if (p > za) {  // the cells of plane p - 1 have all their populations now
@@ -566,12 +700,12 @@ __device__ __forceinline__ void pair_beta(const PairSlots& slots, const Grid& g,
                 static_for<0, Q>([&](auto kc) {
                     constexpr int k = decltype(kc)::value;
                     raw r;
-                    if constexpr (dir_z(k) == 1) r = two::template load_at<dir_x(k), SEP>(sb + k * S::SLOT + dir_y(k) * S::W);
+                    if constexpr (dir_z(k) == 1) r = two::template load_at<dir_x(k)>(sb + k * S::SLOT + dir_y(k) * W, SEP);
                     else if constexpr (dir_z(k) == 0) r = c0[z_rank(k)];
                     else r = m1[z_rank(k)];
                     f[opp(k)] = two::widen(r);
                 });
-                cell_rule2<St>(f, lid, wall, inv_tau, lid_u);
+                cell_rule2<St>(f, lid, wall, ctx.inv_tau, ctx.lid_u);
                 uint32_t ha = 0, hb = 0;
                 if constexpr (St::stochastic) {
                     const uint32_t rh = sr_hash((uint32_t)g.ref(0, y, p - 1), step + 1);
@@ -583,7 +717,7 @@ __device__ __forceinline__ void pair_beta(const PairSlots& slots, const Grid& g,
                         constexpr int k = decltype(kc)::value;
                         const raw r = two::narrow(f[k], ha, hb, k);
                         bits* const q = reinterpret_cast<bits*>(slots.push[k] + off);
-                        if constexpr (SEP == 1 && dir_x(k) == 0) {
+                        if constexpr (k16 && dir_x(k) == 0) {
                             __stcs(reinterpret_cast<raw*>(q), r);
                         } else {
                             __stcs(q, two::first(r));
@@ -601,11 +735,11 @@ __device__ __forceinline__ void pair_beta(const PairSlots& slots, const Grid& g,
             static_for<0, Q>([&](auto kc) {
                 constexpr int k = decltype(kc)::value;
                 if constexpr (dir_z(k) == 0) {
-                    c0[z_rank(k)] = two::template load_at<dir_x(k), SEP>(sb + k * S::SLOT + dir_y(k) * S::W);
+                    c0[z_rank(k)] = two::template load_at<dir_x(k)>(sb + k * S::SLOT + dir_y(k) * W, SEP);
                 }
                 if constexpr (dir_z(k) == -1) {
                     m1[z_rank(k)] = m2[z_rank(k)];
-                    m2[z_rank(k)] = two::template load_at<dir_x(k), SEP>(sb + k * S::SLOT + dir_y(k) * S::W);
+                    m2[z_rank(k)] = two::template load_at<dir_x(k)>(sb + k * S::SLOT + dir_y(k) * W, SEP);
                 }
             });
             // slots that only alpha writes: the neighbour they would come from is a wall
@@ -634,15 +768,15 @@ __device__ __forceinline__ void pair_beta(const PairSlots& slots, const Grid& g,
     named_arrive(1 + NST + stage, S::NB + 32);
 }
 
-template <class St, int TX, int TY, int NST>
-__global__ void __launch_bounds__(PairShape<St, TX, TY, NST>::THREADS, 1)
-    pair_step(const __grid_constant__ CUtensorMap map, const __grid_constant__ PairSlots slots, const Grid g,
-              const float inv_tau, const float lid_u, const int lid_y, const int wall_y,
+template <class St, int TX, int TY, int NST, bool BATCH>
+__global__ void __launch_bounds__(PairShape<St, TX, TY, NST, BATCH>::THREADS, 1)
+    pair_step(const __grid_constant__ CUtensorMap map, const __grid_constant__ PairCtx one,
               const uint32_t* __restrict__ step_base, const uint32_t step_off, const PairWork w,
               int* __restrict__ err)
 {
-    using S = PairShape<St, TX, TY, NST>;
+    using S = PairShape<St, TX, TY, NST, BATCH>;
     extern __shared__ __align__(128) unsigned char pair_smem[];
+    __shared__ PairCtx many[BATCH ? kPairContexts : 1];
     auto* const smem = reinterpret_cast<typename St::bits*>(pair_smem);
     uint64_t* const full = reinterpret_cast<uint64_t*>(smem + NST * S::STAGE);
     int* const item_of = reinterpret_cast<int*>(full + NST);
@@ -652,13 +786,11 @@ __global__ void __launch_bounds__(PairShape<St, TX, TY, NST>::THREADS, 1)
     }
     __syncthreads();
     allow_next_step();  // its blocks take the SMs that this one's leave
+    const PairSource<St, TX, TY, BATCH> src{one, many};
     const uint32_t step = step_of<St>(step_base, step_off);
-    if (threadIdx.x < S::NA)
-        pair_alpha<St, TX, TY, NST>(g, inv_tau, lid_u, lid_y, wall_y, w, step, smem, full, item_of, err);
-    else if (threadIdx.x < S::NA + S::NB)
-        pair_beta<St, TX, TY, NST>(slots, g, inv_tau, lid_u, lid_y, wall_y, w, step, smem, item_of);
-    else
-        pair_copy<St, TX, TY, NST>(&map, g, w, smem, full, item_of);
+    if (threadIdx.x < S::NA) pair_alpha<St, TX, TY, NST, BATCH>(src, step, smem, full, item_of, err);
+    else if (threadIdx.x < S::NA + S::NB) pair_beta<St, TX, TY, NST, BATCH>(src, step, smem, item_of);
+    else pair_copy<St, TX, TY, NST, BATCH>(&map, src, w, smem, full, item_of);
 }
 
 }  // namespace lbm
