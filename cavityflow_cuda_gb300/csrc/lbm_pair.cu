@@ -131,7 +131,7 @@ cudaError_t launch_one(const void* in, void* out, const Grid& g, const Params& p
 }
 
 // Microseconds of a plane of a block with full tiles of 64 cells, GB300.
-constexpr double kPlane[5] = {0, 1.80, 1.70, 1.67, 1.96};
+constexpr double kPlane[5] = {0, 1.80, 1.60, 1.58, 1.81};
 
 // Tiles for a domain of a batch (FP32): the shape whose planes of the whole
 // domain take the least time.  A plane's time, fitted to 45 shapes from 12 x 32
@@ -320,15 +320,19 @@ bool pair_step_pays(int storage, const Grid& g)
     if (sms < 1) return false;
     const Split s = split(g, eb, sms);
     if (s.items > (1ll << 30)) return false;
-    // Measured on GB300, microseconds: a plane of a block, and the separate
-    // kernels' cells per microsecond from memory and, while the state fits L2,
-    // from there (the pair kernel works on two arrays and so never does).
+    // Measured on GB300: the separate kernels' cells per microsecond from memory
+    // and, while the state fits L2, at most, from there (the pair kernel works on
+    // two arrays and so never does).  From memory, rows cost the separate kernels
+    // the time of 16 cells more.  Over 120 domains (31 sizes from 112^3 to 380^3,
+    // 64 to 512 cells wide) none got slower by pairs; 8 stay with the separate
+    // kernels that pairs would make 1-5 % faster.
     static const double rate[5] = {0, 43000, 80000, 80000, 79000};
-    static const double rate_l2[5] = {0, 54000, 75000, 75000, 70000};
+    static const double rate_l2[5] = {0, 54000, 84000, 84000, 78000};
     const double state = (double)Q * (double)g.S * eb;
     const double cells = (double)g.nx * g.ny * g.nz;
-    const double separate = 2.0 * cells / (state < 100e6 ? rate_l2 : rate)[storage];
-    return 6.0 + (double)s.planes * kPlane[storage] < 0.97 * separate;
+    const double separate = state < 100e6 ? cells / rate_l2[storage] : cells / rate[storage] * (1.0 + 16.0 / g.nx);
+    const double plane = kPlane[storage] * (storage == 4 && g.nx % 2 ? 1.05 : 1.0);  // odd rows: both paths of their last warp
+    return 6.0 + (double)s.planes * plane < 0.95 * 2.0 * separate;
 }
 
 cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid& g, const Params& p, int lid_y,

@@ -20,8 +20,8 @@
 //      cells one plane above.  They wait in registers until a cell has all 19;
 //      then it collides and pushes population k to slot k at x + c_k of `out`.
 // Slot k of a cell whose neighbour x - c_k is a wall is written by alpha alone
-// (nobody pushes into it): the cell copies it from the stage to `out`.  So
-// `out` gets every slot that a later step reads; slots that no step reads keep
+// (nobody pushes into it): the copying warp takes it from the stage to `out`
+// when beta is done with the plane.  So `out` gets every slot that a later step reads; slots that no step reads keep
 // what they held.  Results are bit-identical to the separate kernels.
 //
 // The three kinds of threads work on different planes at the same time, a ring
@@ -32,11 +32,11 @@
 // rn.f32x2: the same IEEE operation on both cells, half the instructions).
 //
 // Measured on GB300 at 384^3 (ms a pair, separate kernels -> this one): FP32
-// 2.58 -> 1.49 (76.2 GLUP/s; 93 % of the copy bandwidth for the bytes it moves,
-// 1.11x its array in and 1.0x out), BF16S 1.38 -> 1.09 (104 GLUP/s), F16SR
-// 1.41 -> 1.28 (88.8 GLUP/s; its dither is a fifth of its instructions).  The
-// 16-bit storages are bound by issue slots and the FP32 pipe (54-60 % of the
-// slots used), not by memory.
+// 2.58 -> 1.49 (76.1 GLUP/s; 93 % of the copy bandwidth for the bytes it moves,
+// 1.11x its array in and 1.0x out), F16S 1.39 -> 1.05 and BF16S 1.38 -> 1.04 (109
+// GLUP/s), F16SR 1.41 -> 1.20 (94.4 GLUP/s; its dither is a fifth of its
+// instructions).  The 16-bit storages are bound by their instructions (56-63 %
+// of the issue slots used, with 25 warps a SM), not by memory.
 //
 // Batches (FP32): the items of all domains in one launch, the longest first, with
 // the tiles of each domain as they fit it best (batch_dims in lbm_pair.cu) and a
@@ -44,7 +44,7 @@
 // tile's plane takes 2.1 us instead of 1.9, 0.1 of it for 19 copies in place of
 // one and for addresses from shared memory, the rest for rows that start 8 bytes
 // past a sector.  GLUP/s, the separate kernels -> this one: 64 and 512 cavities
-// of 16 .. 96 cells an edge 35.8 -> 43.8 and 34.4 -> 45.0, 76 of 64^3 37 -> 52,
+// of 16 .. 96 cells an edge 35.8 -> 45.7 and 34.3 -> 47.9, 76 of 64^3 37 -> 51,
 // 610 of 32^3 34.7 -> 42.  The 16-bit storages stay with the separate kernels:
 // they move half the bytes and ran at 0.75 .. 1.0 of their speed here.
 #pragma once
@@ -471,6 +471,43 @@ __host__ __device__ constexpr int z_rank(int k)
     return n;
 }
 
+// Slots of a tile's plane p that no beta thread writes, as the neighbour they
+// would come from is a wall: what alpha left in them goes to `out` as it is.  By
+// the copying warp, which has the time, when beta is done with the stage.  Done
+// by beta's threads this took the tiles at the walls a fifth longer (ms a pair
+// at 384^3, then -> now: BF16S 1.105 -> 1.046, F16SR 1.284 -> 1.208; at 256^3
+// 0.343 -> 0.323 and 0.393 -> 0.368), by alpha's even more (1.168, 1.324).
+template <class St, int SLOT>
+__device__ __forceinline__ void pair_walls(const PairCtx& c, const PairDims& d, const typename St::bits* sb, int x0,
+                                           int y0, int p)
+{
+    using bits = typename St::bits;
+    const Grid& g = c.g;
+    const int lane = (int)threadIdx.x & 31;
+    const int nx = min(d.tx, g.nx + 1 - x0), ny = min(d.ty, g.ny + 1 - y0);
+    const bits* const first = sb + d.w + (g.xoff + x0 - pair_column<St>(g, x0));
+    const uint32_t off = (uint32_t)(g.idx(x0, y0, p) * (long long)sizeof(bits)), row = (uint32_t)(g.P * (long long)sizeof(bits));
+    // columns x .. x + n - 1 of the tile's rows y .. y + m - 1
+    auto area = [&](auto face, int x, int n, int y, int m) {
+#pragma unroll 1
+        for (int i = lane; i < n * m; i += 32) {
+            const int yi = y + i / n, xi = x + i % n;
+            const bits* const from = first + yi * d.w + xi;
+            const uint32_t to = off + (uint32_t)yi * row + (uint32_t)(xi * (int)sizeof(bits));
+            static_for<0, Q>([&](auto kc) {
+                constexpr int k = decltype(kc)::value;
+                if constexpr (decltype(face)::at(k)) *reinterpret_cast<bits*>(c.slots.own[k] + to) = from[k * SLOT];
+            });
+        }
+    };
+    if (x0 == 1) area(FromFace<0, 1>{}, 0, 1, 0, ny);
+    if (x0 + nx > g.nx) area(FromFace<0, -1>{}, nx - 1, 1, 0, ny);
+    if (y0 == 1) area(FromFace<1, 1>{}, 0, nx, 0, 1);
+    if (y0 + ny > g.ny) area(FromFace<1, -1>{}, 0, nx, ny - 1, 1);
+    if (p == 1) area(FromFace<2, 1>{}, 0, nx, 0, ny);
+    if (p == g.nz) area(FromFace<2, -1>{}, 0, nx, 0, ny);
+}
+
 // The copying warp: takes items and brings the planes za - 1 .. zb + 1 of each
 // into the stages, as beta gives them back.  item_of[s] tells the others which
 // item stage s holds (one domain: its number; a batch: the block's how-manieth);
@@ -484,6 +521,17 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSour
     const int lane = (int)threadIdx.x & 31;
     const bool lead = lane == 0;
     int stage = 0, used = 0, item = (int)blockIdx.x, seen = 0;
+    // lane s: what stage s holds, and whether the tile's plane has walls beside it
+    bool walls = false;
+    int held = 0, held_x0 = 0, held_y0 = 0, held_p = 0;
+    auto given_back = [&]() {  // waits until beta is done with `stage`
+        named_sync(1 + NST + stage, S::NB + 32);
+        if (!__shfl_sync(0xffffffffu, (int)walls, stage)) return;
+        const int n = __shfl_sync(0xffffffffu, held, stage);
+        pair_walls<St, S::SLOT>(src.at(n), src.dims(n), smem + stage * S::STAGE, __shfl_sync(0xffffffffu, held_x0, stage),
+                                __shfl_sync(0xffffffffu, held_y0, stage), __shfl_sync(0xffffffffu, held_p, stage));
+        __syncwarp();
+    };
     // `in`, `out` and the counters are the previous step's until it is complete; the other threads touch global memory
     // only after this warp's first copy has arrived
     wait_previous_step();
@@ -521,13 +569,22 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSour
         }
         const PairItem it = src.item(n);
         const PairDims dims = src.dims(n);
-        const int col = pair_column<St>(src.at(n).g, it.x0);
+        const Grid& g = src.at(n).g;
+        const int col = pair_column<St>(g, it.x0);
+        const bool edge = it.x0 == 1 || it.y0 == 1 || it.x0 + dims.tx > g.nx || it.y0 + dims.ty > g.ny;
         int next = 0;
 #pragma unroll 1
         for (int p = it.za - 1; p <= it.zb + 1; ++p) {
             if (lead && p == it.zb) next = atomicAdd(&w.next[0], 1);
-            if (used == NST) named_sync(1 + NST + stage, S::NB + 32);
+            if (used == NST) given_back();
             else ++used;
+            if (lane == stage) {
+                held = n;
+                held_x0 = it.x0;
+                held_y0 = it.y0;
+                held_p = p;
+                walls = p >= it.za && p <= it.zb && (edge || p == 1 || p == g.nz);
+            }
             if (lead) {
                 item_of[stage] = n;
                 tma::fence_proxy_async();  // alpha's and beta's accesses to the stage, before the copy overwrites it
@@ -546,8 +603,9 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSour
         }
         item = __shfl_sync(0xffffffffu, next, 0) + (int)gridDim.x;
     }
-    if (used == NST) named_sync(1 + NST + stage, S::NB + 32);
+    if (used == NST) given_back();
     else ++used;
+    if (lane == stage) walls = false;
     if (lead) {
         item_of[stage] = -1;
         tma::mbar_arrive(&full[stage]);
@@ -558,7 +616,7 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSour
     }
     for (int s = 0; s < used; ++s) {  // beta gives back every stage, the last ones to nobody but this warp
         stage = stage + 1 >= used ? 0 : stage + 1;
-        named_sync(1 + NST + stage, S::NB + 32);
+        given_back();
     }
 }
 
@@ -659,7 +717,7 @@ __device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& s
     // The thread's two cells: FP32 half a row apart, so that each access of a warp is runs of 4-byte elements whatever
     // the shift; 16-bit neighbours, one word.
     int SEP = k16 ? 1 : TX / 2, W = pair_row<St>(TX);
-    bool tile = false, vb = false, lid = false, wall = false, edge = false;
+    bool tile = false, vb = false, whole_rows = false, lid = false, wall = false;
     uint32_t off = 0, pitch = 0;  // of (xa, y, p) in a slot, of a plane, bytes
 #pragma unroll 1
     for (;;) {
@@ -683,9 +741,9 @@ __device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& s
             xa = it.x0 + (k16 ? 2 * px : px);
             tile = ry < d.ty && y <= g.ny && xa <= g.nx;
             vb = xa + SEP <= g.nx;
+            whole_rows = !__any_sync(0xffffffffu, tile && !vb);
             lid = y == src.at(item).lid_y;
             wall = y == src.at(item).wall_y;
-            edge = xa == 1 || xa == g.nx || xa + SEP == g.nx || y == 1 || y == g.ny;
             off = (uint32_t)(g.idx(xa, y, p) * (long long)sizeof(bits));
             pitch = (uint32_t)(g.PY * (long long)sizeof(bits));
             own = smem + (ry + 1) * d.w + (g.xoff + xa - pair_column<St>(g, it.x0));
@@ -712,24 +770,28 @@ __device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& s
                     ha = sr_cell(rh, xa);
                     hb = sr_cell(rh, xa + SEP);
                 }
-                if (vb) {
+                // At a row's end the second cell is the wall behind it.  Predicated stores instead of a branch of
+                // their own are 1-8 % faster (FP32; 16-bit, for rows that do not fill their warp), but not with the
+                // dither of F16SR (2-4 % slower).
+                auto push = [&](auto cells) {
+                    constexpr int kCells = decltype(cells)::value;  // 0: as vb says
                     static_for<0, Q>([&](auto kc) {
                         constexpr int k = decltype(kc)::value;
                         const raw r = two::narrow(f[k], ha, hb, k);
                         bits* const q = reinterpret_cast<bits*>(slots.push[k] + off);
+                        const bool second = kCells == 0 ? vb : kCells == 2;
                         if constexpr (k16 && dir_x(k) == 0) {
-                            __stcs(reinterpret_cast<raw*>(q), r);
+                            if (second) __stcs(reinterpret_cast<raw*>(q), r);
+                            else __stcs(q, two::first(r));
                         } else {
                             __stcs(q, two::first(r));
-                            __stcs(q + SEP, two::second(r));
+                            if (second) __stcs(q + SEP, two::second(r));
                         }
                     });
-                } else {
-                    static_for<0, Q>([&](auto kc) {
-                        constexpr int k = decltype(kc)::value;
-                        *reinterpret_cast<bits*>(slots.push[k] + off) = two::first(two::narrow(f[k], ha, hb, k));
-                    });
-                }
+                };
+                using std::integral_constant;
+                if (k16 && (St::stochastic ? vb : whole_rows)) push(integral_constant<int, 2>{});
+                else push(integral_constant<int, St::stochastic ? 1 : 0>{});
             }
             // what beta pulls from this plane for the cells of this plane and of the next
             static_for<0, Q>([&](auto kc) {
@@ -742,25 +804,6 @@ __device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& s
                     m2[z_rank(k)] = two::template load_at<dir_x(k)>(sb + k * S::SLOT + dir_y(k) * W, SEP);
                 }
             });
-            // slots that only alpha writes: the neighbour they would come from is a wall
-            if (p >= za && p <= zb && (edge || p == 1 || p == g.nz)) {
-                auto keep = [&](auto want, bool first, bool second) {
-                    static_for<0, Q>([&](auto kc) {
-                        constexpr int k = decltype(kc)::value;
-                        if constexpr (decltype(want)::at(k)) {
-                            bits* const q = reinterpret_cast<bits*>(slots.own[k] + off);
-                            if (first) q[0] = sb[k * S::SLOT];
-                            if (second) q[SEP] = sb[k * S::SLOT + SEP];
-                        }
-                    });
-                };
-                if (xa == 1) keep(FromFace<0, 1>{}, true, false);
-                if (xa == g.nx || xa + SEP == g.nx) keep(FromFace<0, -1>{}, xa == g.nx, xa + SEP == g.nx);
-                if (y == 1) keep(FromFace<1, 1>{}, true, vb);
-                if (y == g.ny) keep(FromFace<1, -1>{}, true, vb);
-                if (p == 1) keep(FromFace<2, 1>{}, true, vb);
-                if (p == g.nz) keep(FromFace<2, -1>{}, true, vb);
-            }
         }
         named_arrive(1 + NST + stage, S::NB + 32);
         stage = stage + 1 == NST ? 0 : stage + 1;

@@ -102,3 +102,23 @@ def test_chosen_variant_and_capture_keep_single_steps(gpu):
         assert kernel_launches() - before == 8
         b.run(8)
         assert same_bits(a.get_all(), b.get_all())
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16s", "bf16s", "f16sr"])
+def test_pairs_with_odd_rows(gpu, storage):
+    """Rows of an odd number of cells, whose last pair of cells is one cell and
+    the wall, and the wall slots of all six faces."""
+    from cavityflow_cuda_gb300 import kernel_launches
+
+    n = (447, 300, 200)
+    _, itau = orc.tau_of(0.0192, np.float32)
+    start = _state(n, 3)
+    got = []
+    for launches, variant in ((3, {}), (5, {"fast_variant": 13})):  # two steps a pass, single steps
+        with _solver(n, storage, itau, 0.08, "wall", **variant) as s:
+            s.set_all(start)
+            before = kernel_launches()
+            s.run(5)
+            assert kernel_launches() - before == launches
+            got.append(s.get_all())
+    assert same_bits(*got)
