@@ -123,14 +123,6 @@ int lbm_detail::default_variant(int storage, long long cells)
     }
 }
 
-namespace {
-
-
-}  // namespace
-
-
-
-
 
 int* lbm_detail::err_flag(lbm_solver* s)
 {

@@ -23,7 +23,8 @@
 //                  element-aligned pieces (the default for FP32).
 //   beta_fast_pk -- the direct windows for 16-bit storage with two cells'
 //                  populations packed per 32-bit word and paired conversions
-//                  (the default for the 16-bit storages).
+//                  (the default for the 16-bit storages from 1.1 million
+//                  cells on).
 //   batch_step  -- the persistent kernel of a batch of cavities, running the
 //                  same per-thread bodies over a packed domain table.
 //

@@ -294,8 +294,14 @@ int lbm_step_beta_cuboid(lbm_solver* solver, const int32_t origin[3], const int3
 
 /* `steps` time steps, alpha on an even counter and beta on an odd one,
  * replacing the loop of CController<T>::run / computeNextStep
- * (src/CController.cpp:1278-1287, :1407-1412).  Long runs replay a CUDA
- * graph of captured alpha/beta pairs. */
+ * (src/CController.cpp:1278-1287, :1407-1412).  Where it is faster (F32
+ * without fused_multiply_add, 16-bit storages, larger domains) four steps go
+ * as two passes over the populations between their array and a second one,
+ * which the first such run allocates if it takes at most a quarter of the
+ * free memory, and which is given up when another call of the solver finds
+ * too little memory; never on a capturing stream or with a launch variant that
+ * the caller chose.  Otherwise long runs replay a CUDA graph of captured
+ * alpha/beta pairs.  The state is the same either way, bit for bit. */
 int lbm_run(lbm_solver* solver, int64_t steps, void* stream);
 
 /* Waits for all work queued by the solver.  LBM_ERR_TIMEOUT if one of its
@@ -322,12 +328,13 @@ int lbm_selftest_bounded_wait(lbm_solver* solver, int32_t limit_us);
 int lbm_fast_variant_count(void);
 /* Number of register variants (the first variants; the batch kernel's menu). */
 int lbm_register_variant_count(void);
-/* Selects a variant for subsequent steps; LBM_ERR_UNSUPPORTED if it needs more
- * shared memory than this domain allows. */
+/* Selects a variant for every subsequent step (lbm_run's two steps a pass
+ * included); LBM_ERR_UNSUPPORTED if it needs more shared memory than this domain
+ * allows. */
 int lbm_set_fast_variant(lbm_solver* solver, int32_t variant);
 /* Times every variant that fits this solver's domain (`pairs` alpha/beta pairs
  * each, CUDA events; -1 for a variant that does not fit) and selects the
- * fastest.  The populations are saved to a
+ * fastest for the steps taken one by one.  The populations are saved to a
  * temporary device buffer first and restored afterwards, so the simulation
  * state and step counter are unchanged.  ms_per_pair (optional) receives one
  * time per variant.  Synchronous. */
@@ -428,8 +435,8 @@ int lbm_write_vtk(lbm_solver* solver, const char* path, const double length[3], 
  * domain is a lid-driven box cavity (obstacle halo, lid plane y = ny) with its
  * own size, 1/tau and lid velocity; all advance the same time steps.  The
  * populations of all domains share one device pool and one persistent kernel
- * launch per step walks a packed table of the domains; long runs replay a
- * CUDA graph.  A domain's results are bit-identical to the same domain run
+ * launch per step (or per two, lbm_batch_run) walks a packed table of the
+ * domains; long runs replay a CUDA graph.  A domain's results are bit-identical to the same domain run
  * alone by an lbm_solver of the same storage. */
 typedef struct lbm_batch lbm_batch;   /* opaque */
 
@@ -464,11 +471,13 @@ int lbm_batch_get_info(const lbm_batch* batch, lbm_batch_info* info);
  * not step it alone: lbm_batch_run refuses a batch whose domains have left
  * its time level. */
 int lbm_batch_domain(lbm_batch* batch, int32_t index, lbm_solver** view);
-/* `steps` steps of every domain (alpha on even counters, beta on odd). */
+/* `steps` steps of every domain (alpha on even counters, beta on odd).  F32:
+ * two steps a pass where that is faster, with a second pool, on the terms of
+ * lbm_run's second array. */
 int lbm_batch_run(lbm_batch* batch, int64_t steps, void* stream);
 /* Selects a launch variant (a register variant whose vectors are at most 8
  * bytes wide, since batch rows are packed for them; LBM_ERR_UNSUPPORTED
- * otherwise) for the batch kernel. */
+ * otherwise) for the batch kernel and every subsequent step. */
 int lbm_batch_set_fast_variant(lbm_batch* batch, int32_t variant);
 /* Times each register variant on the whole batch (`pairs` alpha/beta pairs,
  * CUDA events), keeps the fastest and restores the populations.  ms_per_pair
