@@ -897,6 +897,35 @@ int lbm_selftest_bounded_wait(lbm_solver* s, int32_t limit_us)
     return lbm_synchronize(s);
 }
 
+int lbm_selftest_pair_steps(lbm_solver* s, int32_t quads, int64_t wait_limit_ns)
+{
+    if (int r = check_solver(s)) return r;
+    if (quads < 0) return fail(LBM_ERR_INVALID_ARGUMENT, "negative count");
+    CK(cudaSetDevice(s->device), "cudaSetDevice");
+    CK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+    if (int r = check_kernel_flag(s)) return r;  // an earlier failure is reported as such
+    if (s->fma || s->lid_y < 0 || s->last_alpha || !lbm::pair_step_runs(s->storage, s->g))
+        return fail(LBM_ERR_UNSUPPORTED, "the two-steps-a-pass kernel does not run on this solver");
+    const size_t bytes = (size_t)lbm::Q * s->g.S * elem_bytes(s->storage);
+    void* second = nullptr;
+    CK(alloc_or_drop_pairs(s, &second, bytes), "cudaMalloc second array");
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < 2 * quads && e == cudaSuccess; ++i) {
+        lbm::Params p = s->p;
+        p.step_base = step_words(s) + 1;
+        p.step_off = (uint32_t)(s->counter + 2 * (i & 1));
+        e = lbm::launch_pair_step(s->storage, i & 1 ? second : s->dd, i & 1 ? s->dd : second, s->g, p, s->lid_y,
+                                  reinterpret_cast<int*>(s->counts + 3), err_flag(s), 0, wait_limit_ns);
+        if (e == cudaSuccess && (i & 1)) s->counter += 4;
+    }
+    s->macros_fresh = false;
+    const cudaError_t es = cudaDeviceSynchronize();
+    cudaFree(second);
+    if (e != cudaSuccess) return cuda_fail(e, "pair step launch");
+    if (es != cudaSuccess) return cuda_fail(es, "pair steps");
+    return check_kernel_flag(s);
+}
+
 int lbm_fast_variant_count(void) { return lbm::kFastVariantCount; }
 int lbm_register_variant_count(void) { return lbm::kRegisterVariants; }
 

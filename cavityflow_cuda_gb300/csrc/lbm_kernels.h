@@ -126,10 +126,12 @@ cudaError_t launch_fast_step(int storage, int variant, bool alpha, void* dd, con
 // Two steps, alpha then beta, in one pass from the populations `in` to `out`, an
 // array of the same layout (lbm_pair.cuh).  F32 (unfused) and the
 // 16-bit storages.  `work` is two device words that are zero between launches.
+// wait_limit_ns: of the kernel's waits for its copies (negative: two seconds).
 cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid& g, const Params& p, int lid_y,
-                             int* work, int* err, cudaStream_t st);
-// Whether that kernel can run on this domain and takes less time than the
-// default alpha and beta kernels.
+                             int* work, int* err, cudaStream_t st, int64_t wait_limit_ns = -1);
+// Whether that kernel can run on this domain, and whether it then takes less
+// time than the default alpha and beta kernels.
+bool pair_step_runs(int storage, const Grid& g);
 bool pair_step_pays(int storage, const Grid& g);
 
 // The same for the domains of a batch.  A plan is made once for a batch; its

@@ -117,7 +117,7 @@ cudaError_t launch(const CUtensorMap& map, const PairCtx& one, const PairWork& w
 
 template <class St>
 cudaError_t launch_one(const void* in, void* out, const Grid& g, const Params& p, int lid_y, int* work, int* err,
-                       cudaStream_t st)
+                       cudaStream_t st, uint64_t limit_ns)
 {
     constexpr int TY = Shape<St>::TY, eb = (int)sizeof(typename St::bits);
     const int sms = sm_count();
@@ -126,7 +126,7 @@ cudaError_t launch_one(const void* in, void* out, const Grid& g, const Params& p
     const Split s = split(g, eb, sms);
     const PairCtx one{g, pair_slots(out, g, eb), {kTX, TY, pair_row<St>(kTX)}, (int)s.tiles_x, (int)s.tiles, s.zc, 0,
                       (float)p.inv_tau, (float)p.lid_u, lid_y, p.wall_y};
-    const PairWork w{(int)s.items, work, nullptr, nullptr, nullptr, nullptr};
+    const PairWork w{(int)s.items, limit_ns, work, nullptr, nullptr, nullptr, nullptr};
     return launch<St, false>(map, one, w, p.step_base, p.step_off, sms, err, st);
 }
 
@@ -281,7 +281,7 @@ cudaError_t launch_batch(const PairBatchPlan& plan, const void* image, bool back
     const int sms = sm_count();
     if (sms < 1) return cudaErrorNotSupported;
     const char* const at = static_cast<const char*>(image);
-    const PairWork w{plan.items, work, reinterpret_cast<const PairDomain*>(at + plan.domains),
+    const PairWork w{plan.items, tma::kWaitLimitNs, work, reinterpret_cast<const PairDomain*>(at + plan.domains),
                      reinterpret_cast<const int*>(at + plan.domain_of),
                      reinterpret_cast<const CUtensorMap*>(at + plan.maps[back ? 1 : 0]), out};
     const CUtensorMap no_map{};
@@ -310,16 +310,21 @@ cudaError_t launch_pair_batch(int storage, const PairBatchPlan& plan, const void
     return launch_batch<F32>(plan, image, back, out, step_base, step_off, work, err, st);
 }
 
-bool pair_step_pays(int storage, const Grid& g)
+bool pair_step_runs(int storage, const Grid& g)
 {
     if (storage < 1 || storage > 4) return false;
     const int eb = storage_elem_bytes(storage);
     // the copies' 16-byte alignment, 32-bit offsets into a slot, 32-bit item numbers
     if (!default_layout(g, eb) || (unsigned long long)g.S * eb >= (1ull << 32) || !encode_fn()) return false;
     const int sms = sm_count();
-    if (sms < 1) return false;
-    const Split s = split(g, eb, sms);
-    if (s.items > (1ll << 30)) return false;
+    return sms >= 1 && split(g, eb, sms).items <= (1ll << 30);
+}
+
+bool pair_step_pays(int storage, const Grid& g)
+{
+    if (!pair_step_runs(storage, g)) return false;
+    const int eb = storage_elem_bytes(storage);
+    const Split s = split(g, eb, sm_count());
     // Measured on GB300: the separate kernels' cells per microsecond from memory
     // and, while the state fits L2, at most, from there (the pair kernel works on
     // two arrays and so never does).  From memory, rows cost the separate kernels
@@ -336,14 +341,15 @@ bool pair_step_pays(int storage, const Grid& g)
 }
 
 cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid& g, const Params& p, int lid_y,
-                             int* work, int* err, cudaStream_t st)
+                             int* work, int* err, cudaStream_t st, int64_t wait_limit_ns)
 {
     add_launches(1);
+    const uint64_t limit = wait_limit_ns < 0 ? tma::kWaitLimitNs : (uint64_t)wait_limit_ns;
     switch (storage) {
-    case 1: return launch_one<F32>(in, out, g, p, lid_y, work, err, st);
-    case 2: return launch_one<F16S>(in, out, g, p, lid_y, work, err, st);
-    case 3: return launch_one<BF16S>(in, out, g, p, lid_y, work, err, st);
-    case 4: return launch_one<F16SR>(in, out, g, p, lid_y, work, err, st);
+    case 1: return launch_one<F32>(in, out, g, p, lid_y, work, err, st, limit);
+    case 2: return launch_one<F16S>(in, out, g, p, lid_y, work, err, st, limit);
+    case 3: return launch_one<BF16S>(in, out, g, p, lid_y, work, err, st, limit);
+    case 4: return launch_one<F16SR>(in, out, g, p, lid_y, work, err, st, limit);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -306,7 +306,7 @@ struct PairShape {
     static constexpr int NA = ((TY + 2) * (TX / 2 + 2) + 31) / 32 * 32;  // alpha threads: pairs of tile rows -1 .. TY, the frame's columns
     static constexpr int NB = TY * (TX / 2);                     // beta threads
     static constexpr int THREADS = NA + NB + 32;                 // and the warp that issues the copies
-    static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(bits) + NST * (sizeof(uint64_t) + sizeof(int));
+    static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(bits) + NST * (sizeof(uint64_t) + 2 * sizeof(int));
     static_assert(NB % 32 == 0, "whole warps");
     static_assert(1 + 2 * NST <= 15, "named barriers");
 };
@@ -387,6 +387,7 @@ struct PairDomain {
 // each other's frames in L2; a block's copies run ahead into its next item.
 struct PairWork {
     int items;
+    uint64_t limit_ns;          // of the wait for a copy
     int* next;                  // [0] items taken beyond the first of each block, [1] blocks done; zero between launches
     const PairDomain* domains;  // batches: the domains, the domain of each item, the copies' maps of each
     const int* domain_of;       // domain's array, the array written to
@@ -436,10 +437,11 @@ struct PairSource {
     }
 };
 
-// Waits until the phase with `parity` of `bar` has completed, at most limit_ns
-// (tma::mbar_wait with the hardware's own wait between the looks).
-__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns)
+// Waits until the phase with `parity` of `bar` has completed; false when
+// limit_ns have passed since its fill was seen to be issued (*issued == parity).
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns, const volatile int* issued)
 {
+    constexpr uint32_t kNap = 100000;  // ns the hardware may suspend the thread
     uint64_t deadline = 0;
     for (;;) {
         uint32_t done;
@@ -448,12 +450,13 @@ __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, uint64
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done)
-            : "r"(tma::smem_addr(bar)), "r"(parity), "r"(100000u)  // ns the hardware may suspend the thread
+            : "r"(tma::smem_addr(bar)), "r"(parity), "r"(limit_ns < kNap ? (uint32_t)limit_ns : kNap)
             : "memory");
         if (done) return true;
+        if (*issued != (int)parity) continue;
         const uint64_t now = tma::now_ns();
         if (deadline == 0) deadline = now + limit_ns;
-        else if (now > deadline) return false;
+        if (now >= deadline) return false;
     }
 }
 
@@ -511,79 +514,126 @@ __device__ __forceinline__ void pair_walls(const PairCtx& c, const PairDims& d, 
 // The copying warp: takes items and brings the planes za - 1 .. zb + 1 of each
 // into the stages, as beta gives them back.  item_of[s] tells the others which
 // item stage s holds (one domain: its number; a batch: the block's how-manieth);
-// -1 ends the block.
+// -1 ends the block.  Fills of stages are counted over the block's life; fill u
+// goes into stage u % NST; issued[s] is the parity of u / NST of the last one under
+// way or done there.
+//
+// A block also ends when alpha's wait for a copy runs out: alpha then writes -1
+// over the item of that fill, so that all leave at it as at the regular end,
+// without another look at the stages or another store to `out`, and this warp
+// waits, again bounded, for the copies that are still on their way here.  Alpha's
+// clock runs from the issue of the fill: what comes before that, the previous
+// kernel's end or beta giving the stage back, is no fault of the copy, and only
+// then are all through with the stage's last use, so that nobody reads the -1 for
+// another fill or arrives twice on one of its barriers.
 template <class St, int TX, int TY, int NST, bool BATCH>
 __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSource<St, TX, TY, BATCH>& src,
-                                          const PairWork& w, typename St::bits* smem, uint64_t* full, int* item_of)
+                                          const PairWork& w, typename St::bits* smem, uint64_t* full, int* item_of,
+                                          volatile int* issued)
 {
     using S = PairShape<St, TX, TY, NST, BATCH>;
     using bits = typename St::bits;
     const int lane = (int)threadIdx.x & 31;
     const bool lead = lane == 0;
-    int stage = 0, used = 0, item = (int)blockIdx.x, seen = 0;
+    int stage = 0, item = (int)blockIdx.x, next = 0, seen = -1;
     // lane s: what stage s holds, and whether the tile's plane has walls beside it
     bool walls = false;
-    int held = 0, held_x0 = 0, held_y0 = 0, held_p = 0;
-    auto given_back = [&]() {  // waits until beta is done with `stage`
-        named_sync(1 + NST + stage, S::NB + 32);
-        if (!__shfl_sync(0xffffffffu, (int)walls, stage)) return;
-        const int n = __shfl_sync(0xffffffffu, held, stage);
-        pair_walls<St, S::SLOT>(src.at(n), src.dims(n), smem + stage * S::STAGE, __shfl_sync(0xffffffffu, held_x0, stage),
-                                __shfl_sync(0xffffffffu, held_y0, stage), __shfl_sync(0xffffffffu, held_p, stage));
-        __syncwarp();
+    int held_x0 = 0, held_y0 = 0, held_p = 0;
+    // the item whose planes are being brought, the plane that comes next
+    PairItem it{0, 0, 0, -2};
+    PairDims dims{0, 0, 0};
+    int n = 0, p = 0, col = 0, fills = 0, last = -1;
+    uint32_t phase = 0;
+    bool edge = false, all_brought = false;
+    // This block takes no more items.  Every block comes here once, the last one leaves the counters as the next launch
+    // wants them.
+    auto no_more = [&]() {
+        all_brought = true;
+        if (lead && atomicAdd(&w.next[1], 1) == (int)gridDim.x - 1) {
+            w.next[0] = 0;
+            w.next[1] = 0;
+        }
     };
     // `in`, `out` and the counters are the previous step's until it is complete; the other threads touch global memory
     // only after this warp's first copy has arrived
     wait_previous_step();
+    // One turn a fill; after the last, the fill that ends the block, one for each that beta has still to give back.
 #pragma unroll 1
-    while (item < w.items) {
-        const int n = BATCH ? seen++ : item;
-        if constexpr (BATCH) {
-            const int dom = w.domain_of[item];
-            const PairDomain& d = w.domains[dom];
-            PairCtx& c = src.many[n & (kPairContexts - 1)];
-            const Grid g = d.g;
-            static_for<0, Q>([&](auto kc) {
-                constexpr int k = decltype(kc)::value;
-                if (lane == k) {
-                    char* const own = static_cast<char*>(w.out) + (d.offset + k * g.S) * (long long)sizeof(bits);
-                    c.slots.own[k] = own;
-                    c.slots.push[k] = own + ((dir_z(k) - 1) * g.PY + dir_y(k) * g.P + dir_x(k)) * (long long)sizeof(bits);
+    for (int use = 0;; ++use) {
+        if (!all_brought && p == it.zb + 2) {  // the next item, while beta is still busy
+            if (use > 0) item = __shfl_sync(0xffffffffu, next, 0) + (int)gridDim.x;
+            if (item < w.items) {
+                n = BATCH ? ++seen : item;
+                if constexpr (BATCH) {
+                    const int dom = w.domain_of[item];
+                    const PairDomain& d = w.domains[dom];
+                    PairCtx& c = src.many[n & (kPairContexts - 1)];
+                    const Grid g = d.g;
+                    static_for<0, Q>([&](auto kc) {
+                        constexpr int k = decltype(kc)::value;
+                        if (lane == k) {
+                            char* const own = static_cast<char*>(w.out) + (d.offset + k * g.S) * (long long)sizeof(bits);
+                            c.slots.own[k] = own;
+                            c.slots.push[k] =
+                                own + ((dir_z(k) - 1) * g.PY + dir_y(k) * g.P + dir_x(k)) * (long long)sizeof(bits);
+                        }
+                    });
+                    if (lane == Q) {
+                        c.g = g;
+                        c.dims = d.dims;
+                        c.tiles_x = d.tiles_x;
+                        c.tiles = d.tiles;
+                        c.zc = d.zc;
+                        c.item = item - d.item0;
+                        c.inv_tau = d.inv_tau;
+                        c.lid_u = d.lid_u;
+                        c.lid_y = d.lid_y;
+                        c.wall_y = d.wall_y;
+                    }
+                    __syncwarp();
+                    map = w.maps + dom;
+                    if (lead) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
                 }
-            });
-            if (lane == Q) {
-                c.g = g;
-                c.dims = d.dims;
-                c.tiles_x = d.tiles_x;
-                c.tiles = d.tiles;
-                c.zc = d.zc;
-                c.item = item - d.item0;
-                c.inv_tau = d.inv_tau;
-                c.lid_u = d.lid_u;
-                c.lid_y = d.lid_y;
-                c.wall_y = d.wall_y;
+                it = src.item(n);
+                dims = src.dims(n);
+                const Grid& g = src.at(n).g;
+                col = pair_column<St>(g, it.x0);
+                edge = it.x0 == 1 || it.y0 == 1 || it.x0 + dims.tx > g.nx || it.y0 + dims.ty > g.ny;
+                p = it.za - 1;
+            } else {
+                no_more();
+                last = use;
             }
-            __syncwarp();
-            map = w.maps + dom;
-            if (lead) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
         }
-        const PairItem it = src.item(n);
-        const PairDims dims = src.dims(n);
-        const Grid& g = src.at(n).g;
-        const int col = pair_column<St>(g, it.x0);
-        const bool edge = it.x0 == 1 || it.y0 == 1 || it.x0 + dims.tx > g.nx || it.y0 + dims.ty > g.ny;
-        int next = 0;
-#pragma unroll 1
-        for (int p = it.za - 1; p <= it.zb + 1; ++p) {
+        if (use >= NST) {
+            named_sync(1 + NST + stage, S::NB + 32);  // beta is done with fill use - NST
+            const bool at_walls = __shfl_sync(0xffffffffu, (int)walls, stage);
+            const int was = *(const volatile int*)&item_of[stage];
+            if (was < 0) {  // the block ended there
+                if (!all_brought) no_more();
+                for (int u = use - NST; u < fills; ++u)  // copies that nobody has waited for
+                    pair_wait(&full[u % NST], (uint32_t)(u / NST) & 1u, tma::kWaitLimitNs, &issued[u % NST]);
+                return;
+            }
+            if (at_walls) {
+                pair_walls<St, S::SLOT>(src.at(was), src.dims(was), smem + stage * S::STAGE,
+                                        __shfl_sync(0xffffffffu, held_x0, stage), __shfl_sync(0xffffffffu, held_y0, stage),
+                                        __shfl_sync(0xffffffffu, held_p, stage));
+                __syncwarp();
+            }
+        }
+        if (use == last && lead) {
+            item_of[stage] = -1;
+            tma::mbar_arrive(&full[stage]);
+            issued[stage] = (int)phase;
+        }
+        if (!all_brought) {
             if (lead && p == it.zb) next = atomicAdd(&w.next[0], 1);
-            if (used == NST) given_back();
-            else ++used;
             if (lane == stage) {
-                held = n;
                 held_x0 = it.x0;
                 held_y0 = it.y0;
                 held_p = p;
-                walls = p >= it.za && p <= it.zb && (edge || p == 1 || p == g.nz);
+                walls = p >= it.za && p <= it.zb && (edge || p == 1 || p == src.at(n).g.nz);
             }
             if (lead) {
                 item_of[stage] = n;
@@ -598,25 +648,15 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSour
                         "%4, %5}], [%6];" ::"r"(to + (uint32_t)(k * S::SLOT * (int)sizeof(bits))),
                         "l"(map), "r"(col), "r"(it.y0 - 1), "r"(p), "r"(k), "r"(bar)
                         : "memory");
+                issued[stage] = (int)phase;
             }
-            stage = stage + 1 == NST ? 0 : stage + 1;
+            ++p;
+            ++fills;
         }
-        item = __shfl_sync(0xffffffffu, next, 0) + (int)gridDim.x;
-    }
-    if (used == NST) given_back();
-    else ++used;
-    if (lane == stage) walls = false;
-    if (lead) {
-        item_of[stage] = -1;
-        tma::mbar_arrive(&full[stage]);
-        if (atomicAdd(&w.next[1], 1) == (int)gridDim.x - 1) {  // every block has taken its last item
-            w.next[0] = 0;
-            w.next[1] = 0;
+        if (++stage == NST) {
+            stage = 0;
+            phase ^= 1;
         }
-    }
-    for (int s = 0; s < used; ++s) {  // beta gives back every stage, the last ones to nobody but this warp
-        stage = stage + 1 >= used ? 0 : stage + 1;
-        given_back();
     }
 }
 
@@ -624,7 +664,8 @@ __device__ __forceinline__ void pair_copy(const CUtensorMap* map, const PairSour
 template <class St, int TX, int TY, int NST, bool BATCH>
 __device__ __forceinline__ void pair_alpha(const PairSource<St, TX, TY, BATCH>& src, const uint32_t step,
                                            typename St::bits* __restrict__ smem, uint64_t* full,
-                                           const int* item_of, int* __restrict__ err)
+                                           int* item_of, const volatile int* issued, const uint64_t limit_ns,
+                                           int* __restrict__ err)
 {
     using S = PairShape<St, TX, TY, NST, BATCH>;
     using bits = typename St::bits;
@@ -633,16 +674,15 @@ __device__ __forceinline__ void pair_alpha(const PairSource<St, TX, TY, BATCH>& 
     bits* own = smem;
     int stage = 0;
     uint32_t phase = 0;
-    uint64_t limit_ns = tma::kWaitLimitNs;
-    int item = -1, p = 0, y = 0, xa = 0;
+    int item = -2, p = 0, y = 0, xa = 0;  // no item yet
     bool work = false, both = false, lid = false, wall = false;
 #pragma unroll 1
     for (;;) {
         // one warp looks for the copy's arrival, the others sleep in a barrier: 11 or 13 warps looking took
         // issue slots from beta's (F16SR 1.276 ms a pair instead of 1.296 at 384^3)
-        if (tid < 32 && !pair_wait(&full[stage], phase, limit_ns)) {
-            atomicOr(err, 4);  // reported; the block runs on to its end
-            limit_ns = 1000000;
+        if (tid < 32 && !pair_wait(&full[stage], phase, limit_ns, &issued[stage])) {
+            *(volatile int*)&item_of[stage] = -1;
+            atomicOr(err, 4);
         }
         named_sync(1 + 2 * NST, S::NA);
         const int now = *(const volatile int*)&item_of[stage];
@@ -713,7 +753,7 @@ __device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& s
     const int tid = (int)threadIdx.x - S::NA;
     const bits* own = smem;
     raw c0[9], m1[5], m2[5];
-    int stage = 0, item = -1, p = 0, za = 0, zb = 0, y = 0, xa = 0;
+    int stage = 0, item = -2, p = 0, za = 0, zb = 0, y = 0, xa = 0;  // no item yet
     // The thread's two cells: FP32 half a row apart, so that each access of a warp is runs of 4-byte elements whatever
     // the shift; 16-bit neighbours, one word.
     int SEP = k16 ? 1 : TX / 2, W = pair_row<St>(TX);
@@ -825,17 +865,21 @@ __global__ void __launch_bounds__(PairShape<St, TX, TY, NST, BATCH>::THREADS, 1)
     auto* const smem = reinterpret_cast<typename St::bits*>(pair_smem);
     uint64_t* const full = reinterpret_cast<uint64_t*>(smem + NST * S::STAGE);
     int* const item_of = reinterpret_cast<int*>(full + NST);
+    volatile int* const issued = item_of + NST;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NST; ++s) tma::mbar_init(&full[s], 1);
+        for (int s = 0; s < NST; ++s) {
+            tma::mbar_init(&full[s], 1);
+            issued[s] = 1;
+        }
         tma::fence_mbar_init();
     }
     __syncthreads();
     allow_next_step();  // its blocks take the SMs that this one's leave
     const PairSource<St, TX, TY, BATCH> src{one, many};
     const uint32_t step = step_of<St>(step_base, step_off);
-    if (threadIdx.x < S::NA) pair_alpha<St, TX, TY, NST, BATCH>(src, step, smem, full, item_of, err);
+    if (threadIdx.x < S::NA) pair_alpha<St, TX, TY, NST, BATCH>(src, step, smem, full, item_of, issued, w.limit_ns, err);
     else if (threadIdx.x < S::NA + S::NB) pair_beta<St, TX, TY, NST, BATCH>(src, step, smem, item_of);
-    else pair_copy<St, TX, TY, NST, BATCH>(&map, src, w, smem, full, item_of);
+    else pair_copy<St, TX, TY, NST, BATCH>(&map, src, w, smem, full, item_of, issued);
 }
 
 }  // namespace lbm

@@ -111,6 +111,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "lbm_run": ([V, I64, P], I),
         "lbm_synchronize": ([V], I),
         "lbm_selftest_bounded_wait": ([V, C.c_int32], I),
+        "lbm_selftest_pair_steps": ([V, C.c_int32, C.c_int64], I),
         "lbm_fast_variant_count": ([], I),
         "lbm_register_variant_count": ([], I),
         "lbm_set_fast_variant": ([V, C.c_int32], I),

@@ -315,6 +315,14 @@ int lbm_synchronize(lbm_solver* solver);
  * then synchronises.  Returns LBM_ERR_TIMEOUT, after which the solver's
  * state and later steps are unaffected. */
 int lbm_selftest_bounded_wait(lbm_solver* solver, int32_t limit_us);
+/* Diagnostics of lbm_run's kernel that takes two steps a pass: `quads` times
+ * four steps with it on any box cavity that it can run on, also where lbm_run
+ * would not use it, from an even step counter; LBM_ERR_UNSUPPORTED elsewhere.
+ * wait_limit_ns (negative: the usual 2 s) bounds the kernel's waits for its
+ * copies: when one runs out the kernel ends early, the call returns
+ * LBM_ERR_TIMEOUT and the populations are invalid until they are set again.
+ * Uses a second population array while it runs.  Synchronous. */
+int lbm_selftest_pair_steps(lbm_solver* solver, int32_t quads, int64_t wait_limit_ns);
 
 /* ---- tuning (no counterpart in the reference, whose block shape comes from
  * the XML gpu/grid-configuration, src/CConfiguration.cpp:150-160) ---------- */
