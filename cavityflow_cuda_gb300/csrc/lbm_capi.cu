@@ -813,7 +813,7 @@ int lbm_run(lbm_solver* s, int64_t steps, void* stream)
         --left;
     }
     // pairs there and back: the kernels are long enough to need no graph
-    if (steps >= 2 && ensure_pairs(s, st)) {
+    if (left >= 4 && ensure_pairs(s, st)) {
         int* const work = reinterpret_cast<int*>(s->counts + 3);
         lbm::Params p = s->p;
         p.step_base = step_words(s) + 1;

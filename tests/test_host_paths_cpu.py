@@ -1,0 +1,70 @@
+"""The host code around the two-steps-a-pass kernels and the getters, on a
+stand-in for the CUDA runtime (tests/fake/cudart.c) in a process of its own:
+memory that runs out, launches and copies that fail, captures on other streams,
+other threads.  Kernels do nothing there, so these tests say nothing about
+results."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA_INCLUDE = "/usr/local/cuda/include"
+
+PREAMBLE = """
+import ctypes as C, threading, time
+import numpy as np
+from cavityflow_cuda_gb300 import CLbmSolverGB300, LbmBatch, LbmError, LbmServer, kernel_launches
+from cavityflow_cuda_gb300.solver import load_library
+lib = load_library()
+fake = C.CDLL(None)
+fake.fake_used.restype = C.c_size_t
+fake.fake_memory.argtypes = [C.c_size_t]
+fake.fake_live.argtypes = [C.c_void_p]
+fake.fake_capturing.argtypes = [C.c_void_p]
+MB, GB = 1 << 20, 1 << 30
+TIMEOUT = 11
+def solver(n=(256, 256, 256), storage="f32", **kw):
+    return CLbmSolverGB300(n, 1.6, 0.05, storage=storage, **kw)
+def batch(n=(64, 64, 64), count=76, storage="f32"):
+    return LbmBatch([(n, 1.6, 0.05)] * count, storage=storage)
+def run(s, steps):  # launches of a run
+    before = kernel_launches()
+    s.run(steps)
+    return kernel_launches() - before
+LaunchFn = C.CFUNCTYPE(None, C.c_char_p, C.POINTER(C.c_void_p))
+def watch(f):  # f(kernel name, args) before each launch
+    global _cb
+    _cb = LaunchFn(f)
+    fake.fake_on_launch(_cb)
+"""
+
+
+@pytest.fixture(scope="module")
+def child(lib, tmp_path_factory):
+    if not shutil.which("gcc") or not os.path.exists(os.path.join(CUDA_INCLUDE, "cuda_runtime_api.h")):
+        pytest.skip("gcc and the CUDA headers are needed")
+    so = str(tmp_path_factory.mktemp("fake") / "cudart.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-w", "-I" + CUDA_INCLUDE, "-o", so,
+                    os.path.join(HERE, "fake", "cudart.c"), "-lpthread"], check=True)
+
+    def call(code):
+        env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=os.path.dirname(HERE))
+        r = subprocess.run([sys.executable, "-c", PREAMBLE + code], env=env, capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stdout + r.stderr
+
+    return call
+
+
+def test_short_runs_take_no_second_array(child):
+    """Fewer than four steps left, also after a leading beta step, cannot use it."""
+    child("""
+with solver() as s:
+    held = s.info()["device_bytes"]
+    assert [run(s, n) for n in (2, 3, 4, 1)] == [2, 3, 4, 1]   # 4: beta first, three left
+    assert s.info()["device_bytes"] == held
+    assert run(s, 8) == 4                                       # pairs
+    assert s.info()["device_bytes"] > 1.9 * held
+""")
