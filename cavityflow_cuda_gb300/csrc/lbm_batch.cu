@@ -42,6 +42,7 @@ struct lbm_batch {
     size_t pool_bytes = 0;
     std::vector<lbm_solver*> views;
     PackBuffer pack;  // the domains' getters take turns with it
+    BatchFault fault;
     std::vector<lbm::BatchDomain> table;
     lbm::BatchDomain* dtable = nullptr;
     uint32_t* step_words = nullptr;  // [0] first step of a graph replay, [1] zero, [2..3] work words of the pair
@@ -275,6 +276,7 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
     e = cudaMalloc(&b->step_words, 5 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(b->step_words, 0, 5 * sizeof(uint32_t));
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc batch step words"));
+    b->fault.word = reinterpret_cast<int*>(b->step_words + 4);
 
     b->views.reserve((size_t)count);
     for (int i = 0; i < count; ++i) {
@@ -293,7 +295,7 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
         if (r) return bail(r);
         v->batch = b;
         v->batch_pack = &b->pack;
-        v->batch_err = reinterpret_cast<int*>(b->step_words + 4);
+        v->batch_fault = &b->fault;
         b->views.push_back(v);
         r = lbm_set_driven_cavity(v);
         if (r) return bail(r);
@@ -368,7 +370,7 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
     }
     if (left >= 4 && ensure_batch_pairs(b, st)) {
         int* const work = reinterpret_cast<int*>(b->step_words + 2);
-        int* const err = reinterpret_cast<int*>(b->step_words + 4);
+        int* const err = b->fault.word;
         for (; left >= 4; left -= 4)
             for (const bool back : {false, true}) {
                 CK(lbm::launch_pair_batch(b->storage, b->pair_plan, b->pair_image, back, back ? b->pool : b->pool2,

@@ -126,17 +126,25 @@ int lbm_detail::default_variant(int storage, long long cells)
 
 int* lbm_detail::err_flag(lbm_solver* s)
 {
-    return s->batch_err ? s->batch_err : reinterpret_cast<int*>(s->counts + 2);
+    return s->batch_fault ? s->batch_fault->word : reinterpret_cast<int*>(s->counts + 2);
 }
 uint32_t* lbm_detail::step_words(lbm_solver* s) { return reinterpret_cast<uint32_t*>(s->counts + 4); }
 
-// Reads and clears the kernels' timeout flag after the device is idle.
+// Reads and clears the kernels' timeout flag after the device is idle.  A batch's
+// flag counts for each of its domains.
 int lbm_detail::check_kernel_flag(lbm_solver* s)
 {
+    BatchFault* const f = s->batch_fault;
+    std::unique_lock<std::mutex> lock;
+    if (f) lock = std::unique_lock<std::mutex>(f->mutex);
     int flag = 0;
     CK(cudaMemcpy(&flag, err_flag(s), sizeof(int), cudaMemcpyDeviceToHost), "cudaMemcpy error flag");
     if (flag) {
         CK(cudaMemset(err_flag(s), 0, sizeof(int)), "cudaMemset error flag");
+        if (f) ++f->count;
+    }
+    if (flag || (f && s->faults_seen != f->count)) {
+        if (f) s->faults_seen = f->count;
         return fail(LBM_ERR_TIMEOUT, "a step kernel gave up waiting for its bulk copies (flag %d)", flag);
     }
     return LBM_OK;
@@ -337,7 +345,9 @@ int ensure_macros(lbm_solver* s, bool& computed)
 // that ensure_macros computed (`computed`) gave up a wait.
 int check_macros(lbm_solver* s, bool computed)
 {
-    if (!computed || *reinterpret_cast<volatile int*>(s->host_out + 4) == 0) return LBM_OK;
+    const bool raised = *reinterpret_cast<volatile int*>(s->host_out + 4) != 0 ||
+                        (s->batch_fault && s->faults_seen != s->batch_fault->count);
+    if (!computed || !raised) return LBM_OK;
     s->macros_fresh = false;
     return check_kernel_flag(s);
 }

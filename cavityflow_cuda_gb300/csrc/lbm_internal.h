@@ -2,6 +2,7 @@
 // (lbm_capi.cu, lbm_batch.cu); not part of the public interface.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <exception>
 #include <mutex>
@@ -25,6 +26,15 @@ struct PackBuffer {
     bool owned = true;  // false: the end of the solver's macros array
 };
 void free_pack(PackBuffer& b);
+
+// The error flag of a batch's kernels, which step all domains.  The device word
+// is cleared by the first domain that finds it set; `count` is how often that
+// happened, and every domain reports each time once (lbm_solver::faults_seen).
+struct BatchFault {
+    std::mutex mutex;
+    int* word = nullptr;
+    std::atomic<uint64_t> count{0};
+};
 
 }  // namespace lbm_detail
 
@@ -61,7 +71,8 @@ struct lbm_solver {
     int64_t device_bytes = 0;
     bool owns_dd = true;            // false: populations live in a batch's pool
     lbm_batch* batch = nullptr;     // the batch this solver is a domain view of
-    int* batch_err = nullptr;       // the batch's kernel error flag, instead of the solver's
+    lbm_detail::BatchFault* batch_fault = nullptr;  // the batch's kernel error flag, instead of the solver's
+    uint64_t faults_seen = 0;       // of batch_fault->count
 };
 
 namespace lbm_detail {

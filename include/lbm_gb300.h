@@ -477,7 +477,8 @@ int lbm_batch_get_info(const lbm_batch* batch, lbm_batch_info* info);
 /* The solver handle of domain `index`: every single-domain getter, setter and
  * lbm_reduce works on it.  Owned by the batch (lbm_destroy refuses it).  Do
  * not step it alone: lbm_batch_run refuses a batch whose domains have left
- * its time level. */
+ * its time level.  A kernel of the batch that gave up a bounded device-side
+ * wait is reported (LBM_ERR_TIMEOUT) by every domain, once each. */
 int lbm_batch_domain(lbm_batch* batch, int32_t index, lbm_solver** view);
 /* `steps` steps of every domain (alpha on even counters, beta on odd).  F32:
  * two steps a pass where that is faster, with a second pool, on the terms of

@@ -68,3 +68,22 @@ with solver() as s:
     assert run(s, 8) == 4                                       # pairs
     assert s.info()["device_bytes"] > 1.9 * held
 """)
+
+
+def test_every_domain_of_a_batch_reports_an_expired_wait_once(child):
+    """One launch steps all domains, so its failure is each one's."""
+    child("""
+def status(f, *a):
+    try: f(*a)
+    except LbmError as e: return e.status
+    return 0
+with batch((8, 8, 8), 4) as b:
+    v = [b.domain(i) for i in range(4)]
+    b.run(2)
+    assert lib.lbm_selftest_bounded_wait(v[0]._h, 1000) == TIMEOUT      # raises the batch's flag
+    assert status(v[1].getDensities) == TIMEOUT and status(v[1].getDensities) == 0
+    assert lib.lbm_synchronize(v[2]._h) == TIMEOUT and status(v[2].getVelocities) == 0
+    assert lib.lbm_selftest_bounded_wait(v[2]._h, 1000) == TIMEOUT
+    assert [status(x.reduce) for x in v] == [TIMEOUT, TIMEOUT, 0, TIMEOUT]
+    assert [status(x.reduce) for x in v] == [0] * 4
+""")
