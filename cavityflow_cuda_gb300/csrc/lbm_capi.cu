@@ -307,10 +307,9 @@ size_t pack_capacity(const lbm_solver* s)
 }
 
 // Computes the macroscopic fields on the default stream if a step has been taken
-// since (`computed`); check_macros follows once that stream is idle.
-int ensure_macros(lbm_solver* s, bool& computed)
+// since; check_macros follows once that stream is idle.
+int ensure_macros(lbm_solver* s)
 {
-    computed = false;
     CK(cudaSetDevice(s->device), "cudaSetDevice");
     if (!s->macros) {
         // the packing buffer in the same allocation, where it fits
@@ -336,18 +335,21 @@ int ensure_macros(lbm_solver* s, bool& computed)
                               reinterpret_cast<int*>(s->host_out + 4), 0),
            "compute_macros launch");
         s->macros_fresh = true;
-        computed = true;
+        s->macros_checked = false;
     }
     return LBM_OK;
 }
 
-// After the default stream is idle: whether the step kernels behind the fields
-// that ensure_macros computed (`computed`) gave up a wait.
-int check_macros(lbm_solver* s, bool computed)
+// After the default stream is idle: whether the step kernels behind fields that
+// no call has checked yet gave up a wait.  A call that fails in between leaves
+// this to the next one.
+int check_macros(lbm_solver* s)
 {
+    if (s->macros_checked) return LBM_OK;
     const bool raised = *reinterpret_cast<volatile int*>(s->host_out + 4) != 0 ||
                         (s->batch_fault && s->faults_seen != s->batch_fault->count);
-    if (!computed || !raised) return LBM_OK;
+    s->macros_checked = true;
+    if (!raised) return LBM_OK;
     s->macros_fresh = false;
     return check_kernel_flag(s);
 }
@@ -1142,8 +1144,7 @@ static int macro_copy(lbm_solver* s, const int32_t* origin, const int32_t* size,
     if (!host) return fail(LBM_ERR_INVALID_ARGUMENT, "host buffer is NULL");
     int3 o, n;
     if (int r = resolve_cuboid(s, origin, size, o, n)) return r;
-    bool computed = false;
-    if (int r = ensure_macros(s, computed)) return r;
+    if (int r = ensure_macros(s)) return r;
     const size_t vb = (size_t)value_bytes(s->storage);
     const size_t cells = (size_t)n.x * n.y * n.z;
     char* const field = static_cast<char*>(s->macros) + (size_t)first * s->g.cells() * vb;
@@ -1152,15 +1153,15 @@ static int macro_copy(lbm_solver* s, const int32_t* origin, const int32_t* size,
         if (packed.get()) {
             CK(lbm::launch_pack_compact((int)vb, field, count, s->g, o, n, packed.get(), 0), "pack_compact launch");
             CK(cudaMemcpy(host, packed.get(), cells * vb * (size_t)count, cudaMemcpyDeviceToHost), "cudaMemcpy macros");
-            return check_macros(s, computed);
+            return check_macros(s);
         }
     }
     for (int c = 0; c < count; ++c) {
         char* h = static_cast<char*>(host) + (size_t)c * cells * vb;
         CK(copy_compact(field + (size_t)c * s->g.cells() * vb, vb, s->g, o, n, h, to_host), "cudaMemcpy3D macros");
     }
-    if (computed) CK(cudaStreamSynchronize(0), "cudaStreamSynchronize");
-    return check_macros(s, computed);
+    if (!s->macros_checked) CK(cudaStreamSynchronize(0), "cudaStreamSynchronize");
+    return check_macros(s);
 }
 
 int lbm_get_velocities(lbm_solver* s, const int32_t origin[3], const int32_t size[3], void* host)

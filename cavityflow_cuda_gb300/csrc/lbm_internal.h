@@ -48,6 +48,7 @@ struct lbm_solver {
     uint8_t* flags = nullptr;       // one byte per cell, reference layout
     void* macros = nullptr;         // 4 * cells values (rho, jx, jy, jz)
     bool macros_fresh = false;
+    bool macros_checked = true;     // the error flag that came with them has been looked at
     double* scratch = nullptr;      // reduction partials (4 per block) + result (4)
     unsigned long long* counts = nullptr;  // cavity-flag check counters [0..1], kernel error flag [2],
                                            // work words of the pair kernel [3], step words [4] (see step_words)

@@ -87,3 +87,27 @@ with batch((8, 8, 8), 4) as b:
     assert [status(x.reduce) for x in v] == [TIMEOUT, TIMEOUT, 0, TIMEOUT]
     assert [status(x.reduce) for x in v] == [0] * 4
 """)
+
+
+@pytest.mark.parametrize("packed", [True, False])
+def test_failed_copy_does_not_hide_an_expired_wait(child, packed):
+    """The flag comes with the fields; a getter that fails after computing them leaves it to the next one."""
+    child(f"packed = {packed}" + """
+n = (20, 14, 11)
+with solver(n) as s:
+    err = []
+    def steps_fail(name, args):  # the step kernel's work ends with its flag set
+        if err and b"beta" in name: C.c_int.from_address(err[0]).value = 4
+        if b"compute_macros" in name and not err:  # (..., err, host_err)
+            err.append(C.c_void_p.from_address(args[6]).value)
+    watch(steps_fail)
+    s.getDensities()
+    s.run(2)
+    if not packed: fake.fake_memory(0)
+    status = []
+    for i in range(4):  # the runtime keeps a failed copy's error for the next launch to return
+        fake.fake_fail_copies(1 if i == 0 else 0)
+        try: s.getVelocities(); status.append(0)
+        except LbmError as e: status.append(e.status)
+    assert status == [3, 3, TIMEOUT, 0], status
+""")
