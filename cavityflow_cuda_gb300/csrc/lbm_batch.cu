@@ -371,14 +371,24 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
     if (left >= 4 && ensure_batch_pairs(b, st)) {
         int* const work = reinterpret_cast<int*>(b->step_words + 2);
         int* const err = b->fault.word;
-        for (; left >= 4; left -= 4)
-            for (const bool back : {false, true}) {
-                CK(lbm::launch_pair_batch(b->storage, b->pair_plan, b->pair_image, back, back ? b->pool : b->pool2,
-                                          b->step_words + 1, (uint32_t)b->counter, work, err, st),
-                   "batch pair step launch");
-                b->counter += 2;
-                b->last_alpha = false;
+        // the pool is four steps on when both launches are queued; until then it holds the state before them
+        for (; left >= 4 && r == LBM_OK; left -= 4) {
+            cudaError_t e = cudaSuccess;
+            for (const bool back : {false, true})
+                if (e == cudaSuccess)
+                    e = lbm::launch_pair_batch(b->storage, b->pair_plan, b->pair_image, back, back ? b->pool : b->pool2,
+                                               b->step_words + 1, (uint32_t)(b->counter + (back ? 2 : 0)), work, err, st);
+            if (e != cudaSuccess) {
+                r = cuda_fail(e, "batch pair step launch");
+                break;
             }
+            b->counter += 4;
+            b->last_alpha = false;
+        }
+        if (r != LBM_OK) {
+            sync_views(b);
+            return r;
+        }
     }
     const int64_t per_graph = 2 * kBatchGraphPairs;
     if (left >= per_graph) {

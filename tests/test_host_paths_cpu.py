@@ -111,3 +111,20 @@ with solver(n) as s:
         except LbmError as e: status.append(e.status)
     assert status == [3, 3, TIMEOUT, 0], status
 """)
+
+
+@pytest.mark.parametrize("at", [1, 2, 4])
+def test_failed_pair_launch_leaves_a_batch_at_its_last_whole_step(child, at):
+    """After the first of two passes the state is in the second pool only: the step counter counts both or none, and
+    the domains stay at the batch's time level."""
+    child(f"at = {at}" + """
+with batch() as b:
+    b.run(1)
+    fake.fake_fail_launch(b"pair_step", at)
+    try: b.run(17); status = 0
+    except LbmError as e: status = e.status
+    done = 2 + (at - 1) // 2 * 4
+    assert status == 3 and b.info()["step_counter"] == done
+    assert [b.domain(i).info()["step_counter"] for i in (0, 75)] == [done] * 2
+    assert run(b, 8) == 4 and b.info()["step_counter"] == done + 8
+""")
