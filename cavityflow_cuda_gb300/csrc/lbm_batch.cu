@@ -53,7 +53,7 @@ struct lbm_batch {
     bool pairs_refused = false;      // no memory for the second pool
     void* pool2 = nullptr;
     void* pair_image = nullptr;      // the plan's image
-    std::mutex pair_mutex;           // views may give the second pool up from several threads
+    mutable std::mutex pair_mutex;   // of pool2 and pair_image: held while they are made, given up, or launched with
     long long vblocks[2] = {0, 0};  // virtual blocks of the alpha and the beta kernel
     int* vb_map[2] = {nullptr, nullptr};  // domain of each virtual block, per kernel
     long long vb_cap[2] = {0, 0};
@@ -86,9 +86,12 @@ void free_batch_pairs(lbm_batch* b)
 // returns.  The second pool is allocated by the first run that can use it, if
 // it takes at most a quarter of the free memory: the batch could do without
 // it.  A capturing stream gets the separate kernels: the caller's graph must not
-// hold an array that the batch may give up.
-bool ensure_batch_pairs(lbm_batch* b, cudaStream_t st)
+// hold an array that the batch may give up.  `lock` is the caller's until its
+// launches are queued (a view on another thread may give the pool up; cudaFree
+// then waits for them).
+bool ensure_batch_pairs(lbm_batch* b, cudaStream_t st, std::unique_lock<std::mutex>& lock)
 {
+    lock.lock();
     if (!b->pairs || b->pairs_refused) return false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
@@ -105,7 +108,6 @@ bool ensure_batch_pairs(lbm_batch* b, cudaStream_t st)
         b->pair_planned = true;
     }
     if (b->pair_plan.items == 0) return false;
-    std::lock_guard<std::mutex> lock(b->pair_mutex);
     if (b->pool2) return true;
     size_t free_b = 0, total_b = 0;
     const size_t image = b->pair_plan.image.size();
@@ -333,7 +335,10 @@ int lbm_batch_get_info(const lbm_batch* b, lbm_batch_info* info)
                     (int64_t)((b->vb_cap[0] + b->vb_cap[1]) * (long long)sizeof(int));
     for (const lbm_solver* v : b->views) bytes += v->device_bytes;
     bytes += (int64_t)b->pack.bytes;
-    if (b->pool2) bytes += (int64_t)(b->pool_bytes + b->pair_plan.image.size());
+    {
+        std::lock_guard<std::mutex> lock(b->pair_mutex);
+        if (b->pool2) bytes += (int64_t)(b->pool_bytes + b->pair_plan.image.size());
+    }
     info->device_bytes = bytes;
     return LBM_OK;
 }
@@ -368,7 +373,8 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
         if ((r = one(false))) return r;
         --left;
     }
-    if (left >= 4 && ensure_batch_pairs(b, st)) {
+    std::unique_lock<std::mutex> pair_lock(b->pair_mutex, std::defer_lock);
+    if (left >= 4 && ensure_batch_pairs(b, st, pair_lock)) {
         int* const work = reinterpret_cast<int*>(b->step_words + 2);
         int* const err = b->fault.word;
         // the pool is four steps on when both launches are queued; until then it holds the state before them
@@ -390,6 +396,7 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
             return r;
         }
     }
+    if (pair_lock.owns_lock()) pair_lock.unlock();
     const int64_t per_graph = 2 * kBatchGraphPairs;
     if (left >= per_graph) {
         if (!b->graph) {

@@ -128,3 +128,35 @@ with batch() as b:
     assert [b.domain(i).info()["step_counter"] for i in (0, 75)] == [done] * 2
     assert run(b, 8) == 4 and b.info()["step_counter"] == done + 8
 """)
+
+
+def test_second_pool_is_not_given_up_between_launches(child):
+    """A domain's getter on another thread runs out of memory while the batch queues its passes: the pool they write to
+    must be there until they are queued."""
+    child("""
+with batch() as b:
+    v = b.domain(3)
+    assert run(b, 4) == 2
+    used, bad, reached = fake.fake_used(), [], threading.Event()
+    def launch(name, args):
+        if b"pair_step" not in name: return
+        reached.set()
+        time.sleep(0.05)
+        # (map, domain, step_base, step_off, work, err); work ends with domains, domain_of, maps, out
+        at = args[4]
+        ptrs = [C.c_void_p.from_address(at + o).value for o in (24, 32, 40, 48)]
+        if not all(fake.fake_live(p) for p in ptrs): bad.append(ptrs)
+    watch(launch)
+    fake.fake_memory(used)                                      # the getter's fields need the second pool's memory
+    def get():
+        reached.wait()
+        v.getDensities()
+    t = threading.Thread(target=get)
+    t.start()
+    assert run(b, 16) == 8
+    t.join()
+    assert not bad
+    fake.fake_on_launch(None)
+    assert fake.fake_used() < used                              # it has been given up
+    assert run(b, 4) == 4
+""")
