@@ -50,10 +50,7 @@ struct lbm_batch {
     lbm::PairBatchPlan pair_plan;    // two steps a pass, between the pool and a second one (ensure_batch_pairs)
     bool pair_planned = false;
     bool pairs = true;               // no launch variant was asked for
-    bool pairs_refused = false;      // no memory for the second pool
-    void* pool2 = nullptr;
-    void* pair_image = nullptr;      // the plan's image
-    mutable std::mutex pair_mutex;   // of pool2 and pair_image: held while they are made, given up, or launched with
+    SecondArray second;              // the second pool and the plan's image
     long long vblocks[2] = {0, 0};  // virtual blocks of the alpha and the beta kernel
     int* vb_map[2] = {nullptr, nullptr};  // domain of each virtual block, per kernel
     long long vb_cap[2] = {0, 0};
@@ -74,25 +71,14 @@ void drop_batch_graph(lbm_batch* b)
     }
 }
 
-void free_batch_pairs(lbm_batch* b)
-{
-    if (b->pool2) cudaFree(b->pool2);
-    if (b->pair_image) cudaFree(b->pair_image);
-    b->pool2 = b->pair_image = nullptr;
-}
-
 // Whether lbm_batch_run takes two steps a pass on `st`: from the pool to the
 // second one and back, so that the state is always in the pool when a call
-// returns.  The second pool is allocated by the first run that can use it, if
-// it takes at most a quarter of the free memory: the batch could do without
-// it.  A capturing stream gets the separate kernels: the caller's graph must not
-// hold an array that the batch may give up.  `lock` is the caller's until its
-// launches are queued (a view on another thread may give the pool up; cudaFree
-// then waits for them).
+// returns.  A capturing stream gets the separate kernels: the caller's graph must
+// not hold an array that the batch may give up.  `lock` is the caller's until its
+// launches are queued.
 bool ensure_batch_pairs(lbm_batch* b, cudaStream_t st, std::unique_lock<std::mutex>& lock)
 {
-    lock.lock();
-    if (!b->pairs || b->pairs_refused) return false;
+    if (!b->pairs) return false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
         cudaGetLastError();
@@ -108,16 +94,15 @@ bool ensure_batch_pairs(lbm_batch* b, cudaStream_t st, std::unique_lock<std::mut
         b->pair_planned = true;
     }
     if (b->pair_plan.items == 0) return false;
-    if (b->pool2) return true;
-    size_t free_b = 0, total_b = 0;
+    lock.lock();
+    if (b->second.p) return true;
     const size_t image = b->pair_plan.image.size();
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || b->pool_bytes > free_b / 4 ||
-        cudaMalloc(&b->pool2, b->pool_bytes) != cudaSuccess || cudaMalloc(&b->pair_image, image) != cudaSuccess ||
-        !lbm::bind_pair_batch(b->storage, b->pool, b->pool2, b->pair_plan) ||
-        cudaMemcpyAsync(b->pair_image, b->pair_plan.image.data(), image, cudaMemcpyHostToDevice, st) != cudaSuccess) {
+    if (!make_second_array(b->second, b->pool_bytes, image)) return false;
+    if (!lbm::bind_pair_batch(b->storage, b->pool, b->second.p, b->pair_plan) ||
+        cudaMemcpyAsync(b->second.image, b->pair_plan.image.data(), image, cudaMemcpyHostToDevice, st) != cudaSuccess) {
         cudaGetLastError();
-        free_batch_pairs(b);
-        b->pairs_refused = true;
+        lock.unlock();
+        give_up_second_array(b->second);
         return false;
     }
     return true;
@@ -150,7 +135,7 @@ int build_table(lbm_batch* b)
             if (b->vb_map[kind]) cudaFree(b->vb_map[kind]);
             b->vb_map[kind] = nullptr;
             b->vb_cap[kind] = 0;
-            CK(cudaMalloc(&b->vb_map[kind], (size_t)b->vblocks[kind] * sizeof(int)), "cudaMalloc batch block map");
+            CK(device_malloc(&b->vb_map[kind], (size_t)b->vblocks[kind] * sizeof(int)), "cudaMalloc batch block map");
             b->vb_cap[kind] = b->vblocks[kind];
         }
         CK(lbm::launch_batch_map(b->dtable, (int)b->views.size(), b->vblocks[kind], kind, b->vb_map[kind], 0),
@@ -195,21 +180,12 @@ void free_batch(lbm_batch* b)
         if (b->vb_map[kind]) cudaFree(b->vb_map[kind]);
     if (b->step_words) cudaFree(b->step_words);
     free_pack(b->pack);
-    free_batch_pairs(b);
+    remove_second_array(b->second);
     if (b->pool) cudaFree(b->pool);
     delete b;
 }
 
 }  // namespace
-
-bool lbm_detail::drop_batch_pairs(lbm_batch* b)
-{
-    std::lock_guard<std::mutex> lock(b->pair_mutex);
-    if (!b->pool2) return false;
-    free_batch_pairs(b);
-    b->pairs_refused = true;
-    return true;
-}
 
 extern "C" {
 
@@ -247,6 +223,7 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
     b->storage = storage;
     b->device = device;
     b->variant = default_batch_variant(storage);
+    add_second_array(b->second, device);
     auto bail = [&](int r) { free_batch(b); return r; };
 
     // pool layout: each domain's 19 padded slots, 256-byte aligned
@@ -269,13 +246,13 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
         b->interior_cells += (long long)g.nx * g.ny * g.nz;
     }
     b->pool_bytes = elems * (size_t)eb;
-    cudaError_t e = cudaMalloc(&b->pool, b->pool_bytes);
+    cudaError_t e = device_malloc(&b->pool, b->pool_bytes);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc batch pool"));
-    e = cudaMalloc(&b->dtable, (size_t)count * sizeof(lbm::BatchDomain));
+    e = device_malloc(&b->dtable, (size_t)count * sizeof(lbm::BatchDomain));
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc batch table"));
     e = cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
-    e = cudaMalloc(&b->step_words, 5 * sizeof(uint32_t));
+    e = device_malloc(&b->step_words, 5 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(b->step_words, 0, 5 * sizeof(uint32_t));
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc batch step words"));
     b->fault.word = reinterpret_cast<int*>(b->step_words + 4);
@@ -336,8 +313,8 @@ int lbm_batch_get_info(const lbm_batch* b, lbm_batch_info* info)
     for (const lbm_solver* v : b->views) bytes += v->device_bytes;
     bytes += (int64_t)b->pack.bytes;
     {
-        std::lock_guard<std::mutex> lock(b->pair_mutex);
-        if (b->pool2) bytes += (int64_t)(b->pool_bytes + b->pair_plan.image.size());
+        std::lock_guard<std::mutex> lock(b->second.mutex);
+        bytes += (int64_t)b->second.bytes;
     }
     info->device_bytes = bytes;
     return LBM_OK;
@@ -373,8 +350,8 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
         if ((r = one(false))) return r;
         --left;
     }
-    std::unique_lock<std::mutex> pair_lock(b->pair_mutex, std::defer_lock);
-    if (left >= 4 && ensure_batch_pairs(b, st, pair_lock)) {
+    std::unique_lock<std::mutex> second_lock(b->second.mutex, std::defer_lock);
+    if (left >= 4 && ensure_batch_pairs(b, st, second_lock)) {
         int* const work = reinterpret_cast<int*>(b->step_words + 2);
         int* const err = b->fault.word;
         // the pool is four steps on when both launches are queued; until then it holds the state before them
@@ -382,7 +359,7 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
             cudaError_t e = cudaSuccess;
             for (const bool back : {false, true})
                 if (e == cudaSuccess)
-                    e = lbm::launch_pair_batch(b->storage, b->pair_plan, b->pair_image, back, back ? b->pool : b->pool2,
+                    e = lbm::launch_pair_batch(b->storage, b->pair_plan, b->second.image, back, back ? b->pool : b->second.p,
                                                b->step_words + 1, (uint32_t)(b->counter + (back ? 2 : 0)), work, err, st);
             if (e != cudaSuccess) {
                 r = cuda_fail(e, "batch pair step launch");
@@ -396,7 +373,7 @@ int lbm_batch_run(lbm_batch* b, int64_t steps, void* stream)
             return r;
         }
     }
-    if (pair_lock.owns_lock()) pair_lock.unlock();
+    if (second_lock.owns_lock()) second_lock.unlock();
     const int64_t per_graph = 2 * kBatchGraphPairs;
     if (left >= per_graph) {
         if (!b->graph) {
@@ -446,6 +423,7 @@ int lbm_batch_set_fast_variant(lbm_batch* b, int32_t variant)
         return fail(LBM_ERR_UNSUPPORTED, "variant %d's vectors do not fit the batch's packed rows", variant);
     CK(cudaSetDevice(b->device), "cudaSetDevice");
     b->pairs = false;  // every step with the variant asked for
+    give_up_second_array(b->second);
     b->variant = variant;
     for (lbm_solver* v : b->views) v->variant = variant;
     return build_table(b);
@@ -458,12 +436,7 @@ int lbm_batch_autotune(lbm_batch* b, int32_t pairs, int32_t* best, float* ms_per
     CK(cudaSetDevice(b->device), "cudaSetDevice");
     CK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     void* saved = nullptr;
-    cudaError_t es = cudaMalloc(&saved, b->pool_bytes);
-    if (es == cudaErrorMemoryAllocation && drop_batch_pairs(b)) {
-        cudaGetLastError();
-        es = cudaMalloc(&saved, b->pool_bytes);
-    }
-    CK(es, "cudaMalloc autotune snapshot");
+    CK(device_malloc(&saved, b->pool_bytes), "cudaMalloc autotune snapshot");
     cudaStream_t st = b->capture_stream;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     const int start_variant = b->variant;

@@ -241,58 +241,22 @@ int step(lbm_solver* s, bool alpha, const int32_t* origin, const int32_t* size, 
     return LBM_OK;
 }
 
-void drop_pairs(lbm_solver* s)
-{
-    if (!s->dd2) return;
-    cudaFree(s->dd2);
-    s->dd2 = nullptr;
-    s->device_bytes -= (int64_t)((size_t)lbm::Q * s->g.S * elem_bytes(s->storage));
-}
-
-// cudaMalloc that gives up the second population array of lbm_run (or of the
-// batch's runs) rather than fail.
-cudaError_t alloc_or_drop_pairs(lbm_solver* s, void** p, size_t bytes)
-{
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && s->dd2) {
-        cudaGetLastError();
-        drop_pairs(s);
-        s->pairs_refused = true;
-        e = cudaMalloc(p, bytes);
-    } else if (e == cudaErrorMemoryAllocation && s->batch && drop_batch_pairs(s->batch)) {
-        cudaGetLastError();
-        e = cudaMalloc(p, bytes);
-    }
-    return e;
-}
-
 // Whether lbm_run takes two steps a pass on `st` (launch_pair_step, between dd
-// and dd2 and back, so that the state is always in dd when a call returns).
-// The second array is allocated on first use, and only while it is at most a
-// quarter of the free memory, so that a solver which fills the card keeps what
-// it could do without it.  A capturing stream gets the separate kernels: the
-// caller's graph must not hold an array that the solver may give up.
-bool ensure_pairs(lbm_solver* s, cudaStream_t st)
+// and the second array and back, so that the state is always in dd when a call
+// returns).  A capturing stream gets the separate kernels: the caller's graph
+// must not hold an array that the solver may give up.  `lock` is the caller's
+// until its launches are queued.
+bool ensure_pairs(lbm_solver* s, cudaStream_t st, std::unique_lock<std::mutex>& lock)
 {
-    if (!s->pairs || s->pairs_refused || s->fma || s->lid_y < 0 || !s->owns_dd) return false;
+    if (!s->pairs || s->fma || s->lid_y < 0 || !s->owns_dd) return false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     if (capture != cudaStreamCaptureStatusNone || !lbm::pair_step_pays(s->storage, s->g)) return false;
-    if (s->dd2) return true;
-    const size_t bytes = (size_t)lbm::Q * s->g.S * elem_bytes(s->storage);
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 ||
-        cudaMalloc(&s->dd2, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        s->dd2 = nullptr;
-        s->pairs_refused = true;
-        return false;
-    }
-    s->device_bytes += (int64_t)bytes;
-    return true;
+    lock.lock();
+    return make_second_array(s->second, (size_t)lbm::Q * s->g.S * elem_bytes(s->storage), 0);
 }
 
 constexpr size_t kPackBytes = (size_t)96 << 20;  // larger calls copy at the link's rate without packing
@@ -324,7 +288,7 @@ int ensure_macros(lbm_solver* s)
         } else {
             cudaGetLastError();
             s->macros = nullptr;
-            CK(alloc_or_drop_pairs(s, &s->macros, bytes), "cudaMalloc macros");
+            CK(device_malloc(&s->macros, bytes), "cudaMalloc macros");
         }
         s->device_bytes += (int64_t)bytes;
         s->macros_fresh = false;
@@ -463,7 +427,7 @@ int ensure_staging(lbm_solver* s, size_t elems)
         s->staging = nullptr;
         s->staging_elems = 0;
     }
-    CK(alloc_or_drop_pairs(s, (void**)&s->staging, elems * sizeof(float)), "cudaMalloc staging");
+    CK(device_malloc(&s->staging, elems * sizeof(float)), "cudaMalloc staging");
     s->staging_elems = elems;
     s->device_bytes += (int64_t)(elems * sizeof(float));
     return LBM_OK;
@@ -651,12 +615,12 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
     if (external_dd) {
         s->dd = external_dd;
         s->owns_dd = false;
-    } else if ((e = cudaMalloc(&s->dd, dd_bytes)) != cudaSuccess) {
+    } else if ((e = device_malloc(&s->dd, dd_bytes)) != cudaSuccess) {
         return bail(cuda_fail(e, "cudaMalloc populations"));
     }
-    if ((e = cudaMalloc(&s->flags, flag_bytes)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc flags"));
-    if ((e = cudaMalloc(&s->scratch, scratch_bytes)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc scratch"));
-    if ((e = cudaMalloc(&s->counts, 6 * sizeof(unsigned long long))) != cudaSuccess)
+    if ((e = device_malloc(&s->flags, flag_bytes)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc flags"));
+    if ((e = device_malloc(&s->scratch, scratch_bytes)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc scratch"));
+    if ((e = device_malloc(&s->counts, 6 * sizeof(unsigned long long))) != cudaSuccess)
         return bail(cuda_fail(e, "cudaMalloc counters"));
     if ((e = cudaMemset(s->counts, 0, 6 * sizeof(unsigned long long))) != cudaSuccess)
         return bail(cuda_fail(e, "cudaMemset counters"));
@@ -666,6 +630,7 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
         return bail(cuda_fail(e, "cudaMallocHost"));
     if ((e = cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking)) != cudaSuccess)
         return bail(cuda_fail(e, "cudaStreamCreate"));
+    if (s->owns_dd) add_second_array(s->second, s->device);
     s->device_bytes = (int64_t)((s->owns_dd ? dd_bytes : 0) + flag_bytes + scratch_bytes + 16);
 
     lbm::Bc bc;
@@ -699,7 +664,7 @@ void lbm_detail::destroy_solver(lbm_solver* s)
     drop_graph(s);
     if (s->capture_stream) cudaStreamDestroy(s->capture_stream);
     if (s->dd && s->owns_dd) cudaFree(s->dd);
-    if (s->dd2) cudaFree(s->dd2);
+    remove_second_array(s->second);
     free_pack(s->pack);
     if (s->flags) cudaFree(s->flags);
     if (s->macros) cudaFree(s->macros);
@@ -745,7 +710,10 @@ int lbm_get_info(const lbm_solver* s, lbm_info* info)
                                                                             : 0;
     info->row_pitch = s->g.P;
     info->slot_stride = s->g.S;
-    info->device_bytes = s->device_bytes + (int64_t)s->pack.bytes;
+    {
+        std::lock_guard<std::mutex> lock(s->second.mutex);
+        info->device_bytes = s->device_bytes + (int64_t)(s->pack.bytes + s->second.bytes);
+    }
     info->lid_mode = s->lid_mode;
     info->moving_wall = s->p.wall_y > 0 ? 1 : 0;
     info->x1_column = s->g.xoff + 1;
@@ -825,22 +793,24 @@ int lbm_run(lbm_solver* s, int64_t steps, void* stream)
         --left;
     }
     // pairs there and back: the kernels are long enough to need no graph
-    if (left >= 4 && ensure_pairs(s, st)) {
+    std::unique_lock<std::mutex> second_lock(s->second.mutex, std::defer_lock);
+    if (left >= 4 && ensure_pairs(s, st, second_lock)) {
         int* const work = reinterpret_cast<int*>(s->counts + 3);
         lbm::Params p = s->p;
         p.step_base = step_words(s) + 1;
         for (; left >= 4; left -= 4) {
             p.step_off = (uint32_t)s->counter;
-            CK(lbm::launch_pair_step(s->storage, s->dd, s->dd2, s->g, p, s->lid_y, work, err_flag(s), st),
+            CK(lbm::launch_pair_step(s->storage, s->dd, s->second.p, s->g, p, s->lid_y, work, err_flag(s), st),
                "pair step launch");
             p.step_off = (uint32_t)(s->counter + 2);
-            CK(lbm::launch_pair_step(s->storage, s->dd2, s->dd, s->g, p, s->lid_y, work, err_flag(s), st),
+            CK(lbm::launch_pair_step(s->storage, s->second.p, s->dd, s->g, p, s->lid_y, work, err_flag(s), st),
                "pair step launch");
             s->counter += 4;
             s->last_alpha = false;
             s->macros_fresh = false;
         }
     }
+    if (second_lock.owns_lock()) second_lock.unlock();
     const int64_t per_graph = 2 * kGraphPairs;
     if (s->lid_y >= 0 && left >= per_graph) {
         if (!s->graph) {
@@ -920,7 +890,7 @@ int lbm_selftest_pair_steps(lbm_solver* s, int32_t quads, int64_t wait_limit_ns)
         return fail(LBM_ERR_UNSUPPORTED, "the two-steps-a-pass kernel does not run on this solver");
     const size_t bytes = (size_t)lbm::Q * s->g.S * elem_bytes(s->storage);
     void* second = nullptr;
-    CK(alloc_or_drop_pairs(s, &second, bytes), "cudaMalloc second array");
+    CK(device_malloc(&second, bytes), "cudaMalloc second array");
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < 2 * quads && e == cudaSuccess; ++i) {
         lbm::Params p = s->p;
@@ -958,6 +928,7 @@ int lbm_set_fast_variant(lbm_solver* s, int32_t variant)
     if (int r = check_solver(s)) return r;
     if (int r = select_variant(s, variant)) return r;
     s->pairs = false;  // every step with the variant asked for
+    give_up_second_array(s->second);
     return LBM_OK;
 }
 
@@ -970,7 +941,7 @@ int lbm_autotune(lbm_solver* s, int32_t pairs, int32_t* best, float* ms_per_pair
     CK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     const size_t bytes = (size_t)lbm::Q * s->g.S * elem_bytes(s->storage);
     void* saved = nullptr;
-    CK(alloc_or_drop_pairs(s, &saved, bytes), "cudaMalloc autotune snapshot");
+    CK(device_malloc(&saved, bytes), "cudaMalloc autotune snapshot");
     cudaStream_t st = s->capture_stream;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int result = LBM_OK;

@@ -27,6 +27,36 @@ struct PackBuffer {
 };
 void free_pack(PackBuffer& b);
 
+// The second population array of a solver's or a batch's runs that take two steps
+// a pass, and the batch plan's image.  The owner could do without: it is made
+// only while it takes at most a quarter of the free memory, and given up, for
+// good, when an allocation of this library on that device finds too little
+// (lbm_memory.cu).
+struct SecondArray {
+    mutable std::mutex mutex;  // held to read or change what follows, and by a run until its launches are queued
+    void* p = nullptr;
+    void* image = nullptr;
+    size_t bytes = 0;          // of both
+    bool refused = false;      // no memory for it, or given up
+    int device = 0;
+    bool listed = false;
+    SecondArray* prev = nullptr;
+    SecondArray* next = nullptr;
+};
+void add_second_array(SecondArray& a, int device);
+void remove_second_array(SecondArray& a);                            // frees it too
+bool make_second_array(SecondArray& a, size_t bytes, size_t image_bytes);  // a.mutex held; whether it is there
+bool give_up_second_array(SecondArray& a);                           // whether there was one
+bool give_up_any_second_array(int device);
+// cudaMalloc on the current device that gives second arrays up rather than fail.
+// The caller holds no SecondArray's mutex.
+cudaError_t device_malloc(void** p, size_t bytes);
+template <class T>
+cudaError_t device_malloc(T** p, size_t bytes)
+{
+    return device_malloc(reinterpret_cast<void**>(p), bytes);
+}
+
 // The error flag of a batch's kernels, which step all domains.  The device word
 // is cleared by the first domain that finds it set; `count` is how often that
 // happened, and every domain reports each time once (lbm_solver::faults_seen).
@@ -64,9 +94,8 @@ struct lbm_solver {
                                     // while p.wall_y > 0
     lbm_detail::PackBuffer pack;    // the getters' packing buffer
     lbm_detail::PackBuffer* batch_pack = nullptr;  // a batch domain's: shared by the batch
-    void* dd2 = nullptr;            // lbm_run's second population array (ensure_pairs)
+    lbm_detail::SecondArray second; // lbm_run's second population array (ensure_pairs)
     bool pairs = true;              // lbm_run may take two steps a pass: no launch variant was asked for
-    bool pairs_refused = false;     // no memory for dd2
     cudaStream_t capture_stream = nullptr;
     cudaGraphExec_t graph = nullptr;
     int64_t device_bytes = 0;
@@ -92,8 +121,6 @@ int default_batch_variant(int storage);
 // packed rows (see make_grid).
 int create_solver(const lbm_params* prm, void* external_dd, lbm_solver** out, int x1_align = 32, int pitch_align = 0);
 void destroy_solver(lbm_solver* s);
-// Gives back the second pool of a batch; whether there was one.
-bool drop_batch_pairs(lbm_batch* b);
 int* err_flag(lbm_solver* s);
 // Two device words of the solver: [0] the first step of a graph replay,
 // [1] always zero (the base of directly launched steps).

@@ -255,7 +255,7 @@ int upload_table(lbm_server* s, const std::vector<Request*>& reqs, long long (&v
         if (s->dtable) cudaFree(s->dtable);
         s->dtable = nullptr;
         const size_t cap = std::max<size_t>(reqs.size() * 2, 64);
-        CK(cudaMalloc(&s->dtable, cap * sizeof(lbm::BatchDomain)), "cudaMalloc server table");
+        CK(device_malloc(&s->dtable, cap * sizeof(lbm::BatchDomain)), "cudaMalloc server table");
         s->dtable_cap = cap;
     }
     CK(cudaMemcpyAsync(s->dtable, s->table.data(), reqs.size() * sizeof(lbm::BatchDomain), cudaMemcpyHostToDevice,
@@ -268,7 +268,7 @@ int upload_table(lbm_server* s, const std::vector<Request*>& reqs, long long (&v
             s->vb_map[kind] = nullptr;
             s->vb_cap[kind] = 0;
             const long long cap = std::max<long long>(vblocks[kind] + vblocks[kind] / 2, 1024);
-            CK(cudaMalloc(&s->vb_map[kind], (size_t)cap * sizeof(int)), "cudaMalloc server block map");
+            CK(device_malloc(&s->vb_map[kind], (size_t)cap * sizeof(int)), "cudaMalloc server block map");
             s->vb_cap[kind] = cap;
         }
         CK(lbm::launch_batch_map(s->dtable, (int)reqs.size(), vblocks[kind], kind, s->vb_map[kind], s->stream),
@@ -376,14 +376,16 @@ int lbm_server_create(const lbm_server_config* cfg, lbm_server** out)
         return fail(LBM_ERR_UNSUPPORTED, "variant %d's vectors do not fit the server's packed rows", s->variant);
     }
     s->arena_bytes = (size_t)((double)cfg->budget_bytes * kArenaShare) / kAlign * kAlign;
+    while (s->arena_bytes + (size_t)(1 << 30) > free_b && give_up_any_second_array(cfg->device))
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) cudaGetLastError();
     if (s->arena_bytes + (size_t)(1 << 30) > free_b) {
         delete s;
         return fail(LBM_ERR_BUDGET, "budget of %lld bytes exceeds the free device memory (%zu bytes)",
                     (long long)cfg->budget_bytes, free_b);
     }
-    cudaError_t e = cudaMalloc((void**)&s->arena, s->arena_bytes);
+    cudaError_t e = device_malloc(&s->arena, s->arena_bytes);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&s->zero_word, sizeof(uint32_t));
+    if (e == cudaSuccess) e = device_malloc(&s->zero_word, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(s->zero_word, 0, sizeof(uint32_t));
     if (e != cudaSuccess) {
         lbm_server_destroy(s);

@@ -292,16 +292,21 @@ int lbm_step_beta(lbm_solver* solver, void* stream);
 int lbm_step_beta_cuboid(lbm_solver* solver, const int32_t origin[3], const int32_t size[3],
                          void* stream);
 
+/* Two steps a pass: where it is faster (F32 without fused_multiply_add, 16-bit
+ * storages, larger domains; F32 batches) lbm_run and lbm_batch_run take four
+ * steps as two passes over the populations, between their array and a second
+ * one.  The first such run allocates that if it takes at most a quarter of the
+ * free memory; else the solver does without for good.  It is given up, for
+ * good, when any allocation of this library on the device finds too little
+ * memory; a program that needs its memory elsewhere gets it back by
+ * lbm_set_fast_variant (lbm_batch_set_fast_variant).  Never on a capturing
+ * stream, nor with a launch variant that the caller chose. */
+
 /* `steps` time steps, alpha on an even counter and beta on an odd one,
  * replacing the loop of CController<T>::run / computeNextStep
- * (src/CController.cpp:1278-1287, :1407-1412).  Where it is faster (F32
- * without fused_multiply_add, 16-bit storages, larger domains) four steps go
- * as two passes over the populations between their array and a second one,
- * which the first such run allocates if it takes at most a quarter of the
- * free memory, and which is given up when another call of the solver finds
- * too little memory; never on a capturing stream or with a launch variant that
- * the caller chose.  Otherwise long runs replay a CUDA graph of captured
- * alpha/beta pairs.  The state is the same either way, bit for bit. */
+ * (src/CController.cpp:1278-1287, :1407-1412).  Two steps a pass (above), or
+ * else long runs replay a CUDA graph of captured alpha/beta pairs.  The state
+ * is the same either way, bit for bit. */
 int lbm_run(lbm_solver* solver, int64_t steps, void* stream);
 
 /* Waits for all work queued by the solver.  LBM_ERR_TIMEOUT if one of its
@@ -336,9 +341,9 @@ int lbm_selftest_pair_steps(lbm_solver* solver, int32_t quads, int64_t wait_limi
 int lbm_fast_variant_count(void);
 /* Number of register variants (the first variants; the batch kernel's menu). */
 int lbm_register_variant_count(void);
-/* Selects a variant for every subsequent step (lbm_run's two steps a pass
- * included); LBM_ERR_UNSUPPORTED if it needs more shared memory than this domain
- * allows. */
+/* Selects a variant for every subsequent step (lbm_run no longer takes two
+ * steps a pass, and frees its second array); LBM_ERR_UNSUPPORTED if it needs
+ * more shared memory than this domain allows. */
 int lbm_set_fast_variant(lbm_solver* solver, int32_t variant);
 /* Times every variant that fits this solver's domain (`pairs` alpha/beta pairs
  * each, CUDA events; -1 for a variant that does not fit) and selects the
@@ -481,12 +486,12 @@ int lbm_batch_get_info(const lbm_batch* batch, lbm_batch_info* info);
  * wait is reported (LBM_ERR_TIMEOUT) by every domain, once each. */
 int lbm_batch_domain(lbm_batch* batch, int32_t index, lbm_solver** view);
 /* `steps` steps of every domain (alpha on even counters, beta on odd).  F32:
- * two steps a pass where that is faster, with a second pool, on the terms of
- * lbm_run's second array. */
+ * two steps a pass where that is faster, on the terms given at lbm_run. */
 int lbm_batch_run(lbm_batch* batch, int64_t steps, void* stream);
 /* Selects a launch variant (a register variant whose vectors are at most 8
  * bytes wide, since batch rows are packed for them; LBM_ERR_UNSUPPORTED
- * otherwise) for the batch kernel and every subsequent step. */
+ * otherwise) for the batch kernel and every subsequent step, as
+ * lbm_set_fast_variant does. */
 int lbm_batch_set_fast_variant(lbm_batch* batch, int32_t variant);
 /* Times each register variant on the whole batch (`pairs` alpha/beta pairs,
  * CUDA events), keeps the fastest and restores the populations.  ms_per_pair

@@ -160,3 +160,92 @@ with batch() as b:
     assert fake.fake_used() < used                              # it has been given up
     assert run(b, 4) == 4
 """)
+
+
+@pytest.mark.parametrize("other", ["solver", "batch", "server", "fields", "autotune"])
+def test_second_arrays_go_to_whoever_needs_the_memory(child, other):
+    """What could be made before runs took second arrays can still be made after them."""
+    child(f"other = {other!r}" + """
+with solver() as a, batch() as b:
+    half = a.info()["device_bytes"], b.info()["device_bytes"]
+    assert run(a, 8) == 4 and run(b, 8) == 4
+    both = a.info()["device_bytes"], b.info()["device_bytes"]
+    assert both[0] > 1.9 * half[0] and both[1] > 1.5 * half[1]
+    with solver((250, 256, 256)) as c:
+        assert run(c, 4) == 2
+        if other == "solver":
+            fake.fake_memory(fake.fake_used() + 200 * MB)
+            d = solver()
+        elif other == "batch":
+            fake.fake_memory(fake.fake_used() + 200 * MB)
+            d = batch((64, 64, 60), 100)
+        elif other == "server":
+            fake.fake_memory(fake.fake_used() + 200 * MB)
+            d = LbmServer(budget_bytes=2 * GB, storage="f16sr")
+        elif other == "fields":
+            fake.fake_memory(fake.fake_used())
+            a.getDensities(out=np.empty((256, 256, 256), np.float32))
+            d = None
+        else:
+            fake.fake_memory(fake.fake_used())
+            c.autotune(1)
+            d = None
+        held = a.info()["device_bytes"] + b.info()["device_bytes"] + c.info()["device_bytes"]
+        fake.fake_memory(1 << 40)
+        if d: d.close()
+        n = run(a, 8) + run(b, 8) + run(c, 8)
+        assert 12 < n <= 24 and held < 2 * (half[0] + half[1] + half[0])
+assert fake.fake_used() == 0
+""")
+
+
+def test_memory_that_is_nobodys_second_array_still_runs_out(child):
+    child("""
+with solver() as a:
+    run(a, 8)
+    fake.fake_memory(fake.fake_used() + 200 * MB)
+    for make in (lambda: solver((512, 512, 256)), lambda: batch((64, 64, 64), 300),
+                 lambda: LbmServer(budget_bytes=6 * GB, storage="f16sr")):
+        try: make(); status = 0
+        except LbmError as e: status = e.status
+        assert status in (4, 8), status
+    assert run(a, 8) == 8
+""")
+
+
+def test_chosen_variant_gives_the_second_array_back(child):
+    child("""
+for s in (solver(), batch()):
+    held, used = s.info()["device_bytes"], fake.fake_used()
+    assert run(s, 8) == 4 and s.info()["device_bytes"] > held
+    s.set_fast_variant(s.info()["fast_variant"])
+    assert s.info()["device_bytes"] == held and fake.fake_used() == used
+    assert run(s, 8) == 8
+    s.close()
+""")
+
+
+@pytest.mark.parametrize("share,pairs", [(3.9, False), (4.1, True)])
+def test_second_array_takes_at_most_a_quarter_of_the_free_memory(child, share, pairs):
+    child(f"share, pairs = {share}, {pairs}" + """
+for make in (solver, batch):
+    with make() as s:
+        pop = 19 * s.info()["slot_stride"] * 4 if make is solver else 76 * 19 * s.domain(0).info()["slot_stride"] * 4
+        fake.fake_memory(fake.fake_used() + int(share * pop))
+        assert run(s, 8) == (4 if pairs else 8)
+        fake.fake_memory(1 << 40)
+        assert run(s, 8) == (4 if pairs else 8)    # refused for good
+""")
+
+
+def test_capturing_stream_takes_single_steps_and_no_memory(child):
+    child("""
+for make in (solver, batch):
+    with make() as s:
+        used = fake.fake_used()
+        fake.fake_capturing(0x1000)
+        before = kernel_launches()
+        s.run(8, stream=0x1000)
+        assert kernel_launches() - before == 8 and fake.fake_used() == used
+        assert run(s, 8) == 4
+""")
