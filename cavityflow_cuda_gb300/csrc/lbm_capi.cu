@@ -353,6 +353,7 @@ public:
 private:
     bool grow(lbm_solver* s, size_t bytes)
     {
+        const lbm_detail::BesideCaptures beside;
         const size_t want = std::max(bytes, std::min(kPackBytes, pack_capacity(s)));
         if (!b_.idle && cudaEventCreateWithFlags(&b_.idle, cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();

@@ -27,6 +27,21 @@ struct PackBuffer {
 };
 void free_pack(PackBuffer& b);
 
+// Lets this thread allocate and free while a stream is captured elsewhere in
+// global mode, which such calls would otherwise break.  For memory that a call
+// could do without: the calls that take it worked beside a capture when they
+// took none.
+class BesideCaptures {
+public:
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    BesideCaptures(const BesideCaptures&) = delete;
+    BesideCaptures& operator=(const BesideCaptures&) = delete;
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // The second population array of a solver's or a batch's runs that take two steps
 // a pass, and the batch plan's image.  The owner could do without: it is made
 // only while it takes at most a quarter of the free memory, and given up, for

@@ -14,6 +14,7 @@ SecondArray* list = nullptr;
 
 void release(SecondArray& a)
 {
+    const BesideCaptures beside;
     if (a.p || a.image) cudaDeviceSynchronize();  // queued passes still use them
     if (a.p) cudaFree(a.p);
     if (a.image) cudaFree(a.image);
@@ -52,6 +53,7 @@ bool make_second_array(SecondArray& a, size_t bytes, size_t image_bytes)
 {
     if (a.refused) return false;
     if (a.p) return true;
+    const BesideCaptures beside;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 ||
         cudaMalloc(&a.p, bytes) != cudaSuccess ||

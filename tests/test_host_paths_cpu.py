@@ -249,3 +249,22 @@ for make in (solver, batch):
         assert kernel_launches() - before == 8 and fake.fake_used() == used
         assert run(s, 8) == 4
 """)
+
+
+def test_memory_is_taken_without_breaking_a_capture_elsewhere(child):
+    """Runs and the populations' getter took no memory before they took two steps a pass or packed: they still work
+    beside a capture in global mode on another stream."""
+    child("""
+st = 0x2000
+for make in (solver, batch):
+    with make() as s, solver((40, 30, 20)) as t:
+        fake.fake_capture_elsewhere(1)
+        before = kernel_launches()
+        s.run(8, stream=st)
+        assert kernel_launches() - before == 4 and not fake.fake_capture_broken()
+        out = np.empty((19, 20, 30, 40), np.float32)
+        assert lib.lbm_get_density_distributions(t._h, None, None, out.ctypes.data, st) == 0
+        s.set_fast_variant(s.info()["fast_variant"]) if make is solver else None
+        assert not fake.fake_capture_broken()
+        fake.fake_capture_elsewhere(0)
+""")
