@@ -189,7 +189,8 @@ void free_batch(lbm_batch* b)
 
 extern "C" {
 
-static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count, int32_t storage, int32_t device, lbm_batch** out)
+static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count, int32_t storage, int32_t device,
+                                  int pitch_align, lbm_batch** out)
 {
     if (!domains || !out || count <= 0) return fail(LBM_ERR_INVALID_ARGUMENT, "domains, count and out are required");
     *out = nullptr;
@@ -233,7 +234,7 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
     b->table.resize((size_t)count);
     for (int i = 0; i < count; ++i) {
         const lbm::Grid g = lbm::make_grid(domains[i].size[0], domains[i].size[1], domains[i].size[2], eb,
-                                           lbm::kPackedX1Align, lbm::batch_pitch_align(storage));
+                                           lbm::kPackedX1Align, pitch_align);
         offsets[(size_t)i] = elems;
         elems += (size_t)lbm::Q * g.S;  // S keeps every slot 256-byte aligned
         lbm::BatchDomain& d = b->table[(size_t)i];
@@ -270,7 +271,7 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
         p.fast_variant = b->variant + 1;
         lbm_solver* v = nullptr;
         int r = create_solver(&p, static_cast<char*>(b->pool) + offsets[(size_t)i] * (size_t)eb, &v,
-                              lbm::kPackedX1Align, lbm::batch_pitch_align(storage));
+                              lbm::kPackedX1Align, pitch_align);
         if (r) return bail(r);
         v->batch = b;
         v->batch_pack = &b->pack;
@@ -287,7 +288,15 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
 
 int lbm_batch_create(const lbm_domain_spec* domains, int32_t count, int32_t storage, int32_t device, lbm_batch** out)
 {
-    return guarded("lbm_batch_create", [&] { return batch_create_unguarded(domains, count, storage, device, out); });
+    return guarded("lbm_batch_create", [&] {
+        const int align = lbm::batch_pitch_align(storage);
+        const int r = batch_create_unguarded(domains, count, storage, device, align, out);
+        // Without the padding that two steps a pass need (up to 3 % of the pool for rows from 64 cells on, a third for
+        // rows of one or two) the batch may still fit.
+        if (r != LBM_ERR_OUT_OF_MEMORY || align == 0) return r;
+        cudaGetLastError();
+        return batch_create_unguarded(domains, count, storage, device, 0, out);
+    });
 }
 
 int lbm_batch_destroy(lbm_batch* b)

@@ -268,3 +268,23 @@ for make in (solver, batch):
         assert not fake.fake_capture_broken()
         fake.fake_capture_elsewhere(0)
 """)
+
+
+def test_batch_without_room_for_row_padding_keeps_its_narrow_rows(child):
+    """Rows are padded to what two steps a pass need only where the padded pool fits."""
+    child("""
+def pool(b, n, count):
+    return count * 19 * 4 * b.domain(0).info()["slot_stride"]
+for n, count, rows in (((2, 900, 900), 4, (8, 6)), ((64, 64, 64), 76, (68, 68)), ((65, 64, 64), 76, (72, 70))):
+    with batch(n, count) as b:
+        assert b.domain(0).info()["row_pitch"] == rows[0], b.domain(0).info()["row_pitch"]
+        wide, rest = pool(b, n, count), b.info()["device_bytes"] - pool(b, n, count)
+    if rows[0] == rows[1]: continue
+    assert wide * rows[1] // rows[0] + rest < wide - 1
+    fake.fake_memory(wide - 1)
+    with batch(n, count) as b:
+        assert b.domain(0).info()["row_pitch"] == rows[1]
+        assert [b.domain(i).info()["row_pitch"] for i in (1, count - 1)] == [rows[1]] * 2
+        fake.fake_memory(1 << 40)
+        assert run(b, 8) == 8
+""")
