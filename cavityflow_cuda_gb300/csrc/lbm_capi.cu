@@ -112,12 +112,27 @@ int lbm_detail::default_batch_variant(int storage)
 // in a replayed graph, F16SR: 32^3 variant 20 3.95, 6 2.67; 64^3 20 6.23, 6 5.67,
 // 8 5.07; 96^3 20 13.5, 8 12.6, 23 12.5; 112^3 20 19.1, 8 18.8, 23 18.0; 128^3 20
 // 30.2, 23 30.0, 8 34.5; BF16S alike).
-int lbm_detail::default_variant(int storage, long long cells)
+// Rows shorter than 32 cells have limits of their own (measured 3 to 31 wide, 60 000 to 1.9 million cells, all three
+// storages).  Two cells a thread: while the chip holds all blocks, two an SM (BF16S 30 x 71 x 70, 350 blocks: 6 5.49, 20
+// 4.87; 25 x 80 x 80, 400: 6 6.07, 20 5.63, 8 5.02; 25 x 76 x 76, 304: 6 4.34, 8 5.00; 9 x 103 x 102, 306: 6 4.93, 8 5.06).
+// Eight: in rows of two or four 16-byte vectors, once the state, padding included, no longer stays in L2 (F16SR 11 x 369
+// x 369, 230 MB: 23 74.8, 20 68.6; 9 x 333 x 333, 202 MB: 8 59.2, 20 56.6; 26 x 267 x 266, 175 MB: 23 51.5, 20 49.3; 13 x
+// 248 x 248, 114 MB: 8 27.6, 20 26.2; 13 x 196 x 196, 70 MB: 8 11.5, 20 13.8; 9 x 236 x 235, 101 MB: 8 18.5, 20 21.2; 28
+// x 215 x 215, 115 MB: 23 25.2, 20 28.7).  17 .. 24 wide 23 stays ahead by 3 %.
+int lbm_detail::default_variant(int storage, const lbm::Grid& g)
 {
+    const long long cells = (long long)g.nx * g.ny * g.nz;
     switch (storage) {
     case LBM_STORAGE_F16S:
     case LBM_STORAGE_BF16S:
     case LBM_STORAGE_F16SR:
+        if (g.nx < 32) {
+            const long long plane_blocks = ((g.nx + 1) / 2 * (long long)g.ny + 255) / 256;
+            if (cells < 170000 && plane_blocks * g.nz > 310) return 8;
+            const double state = (double)lbm::Q * (double)g.S * 2;
+            const bool half_used = g.nx % 16 >= 9 && g.nx % 16 <= 12;  // the row's last vector
+            if ((half_used && state > 140e6) || (g.nx >= 13 && g.nx <= 16 && state > 110e6)) return 20;
+        }
         return cells < 170000 ? 6 : cells < 1100000 ? 8 : cells < 1900000 ? 23 : 20;
     default: return 13;
     }
@@ -601,7 +616,7 @@ int lbm_detail::create_solver(const lbm_params* prm, void* external_dd, lbm_solv
                     lbm::kFastVariantCount);
     }
     s->variant = prm->fast_variant == 0
-                     ? default_variant(s->storage, (long long)s->g.nx * s->g.ny * s->g.nz)
+                     ? default_variant(s->storage, s->g)
                      : prm->fast_variant - 1;
     s->pairs = prm->fast_variant == 0;
     s->fma = prm->fused_multiply_add == 1;

@@ -126,8 +126,8 @@ int fail(int status, const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 int elem_bytes(int storage);
 int value_bytes(int storage);
-// Default register variant of a domain of that many interior cells.
-int default_variant(int storage, long long cells);
+// Default register variant of a domain.
+int default_variant(int storage, const lbm::Grid& g);
 // Default register variant of the batch kernel (many small domains).
 int default_batch_variant(int storage);
 // Creates a solver; with `external_dd` its populations live there (a batch
