@@ -130,9 +130,6 @@ cudaError_t launch_one(const void* in, void* out, const Grid& g, const Params& p
     return launch<St, false>(map, one, w, p.step_base, p.step_off, sms, err, st);
 }
 
-// Microseconds of a plane of a block with full tiles of 64 cells, GB300.
-constexpr double kPlane[5] = {0, 1.80, 1.60, 1.58, 1.81};
-
 // Tiles for a domain of a batch (FP32): the shape whose planes of the whole
 // domain take the least time.  A plane's time, fitted to 45 shapes from 12 x 32
 // to 128 x 3 (7 % off on average): its cells', and its rows', which a warp's
@@ -323,21 +320,46 @@ bool pair_step_runs(int storage, const Grid& g)
 bool pair_step_pays(int storage, const Grid& g)
 {
     if (!pair_step_runs(storage, g)) return false;
-    const int eb = storage_elem_bytes(storage);
-    const Split s = split(g, eb, sm_count());
-    // Measured on GB300: the separate kernels' cells per microsecond from memory
-    // and, while the state fits L2, at most, from there (the pair kernel works on
-    // two arrays and so never does).  From memory, rows cost the separate kernels
-    // the time of 16 cells more.  Over 120 domains (31 sizes from 112^3 to 380^3,
-    // 64 to 512 cells wide) none got slower by pairs; 8 stay with the separate
-    // kernels that pairs would make 1-5 % faster.
-    static const double rate[5] = {0, 43000, 80000, 80000, 79000};
-    static const double rate_l2[5] = {0, 54000, 84000, 84000, 78000};
-    const double state = (double)Q * (double)g.S * eb;
-    const double cells = (double)g.nx * g.ny * g.nz;
-    const double separate = state < 100e6 ? cells / rate_l2[storage] : cells / rate[storage] * (1.0 + 16.0 / g.nx);
-    const double plane = kPlane[storage] * (storage == 4 && g.nx % 2 ? 1.05 : 1.0);  // odd rows: both paths of their last warp
-    return 6.0 + (double)s.planes * plane < 0.95 * 2.0 * separate;
+    const int eb = storage_elem_bytes(storage), sms = sm_count();
+    // Microseconds of a pair, fitted to 2350 boxes of 0.3 to 30 million cells with axes up to 8 times off the cube's, GB300.
+    //
+    // Separate kernels (2 % off, one standard deviation): cells at a rate from memory and at one from L2, in proportion
+    // while the state is between two sizes; from memory a row costs `row` cells more, and so does what its last vector
+    // leaves unused, everywhere.
+    //
+    // This kernel (4 % off): the busiest block's planes, of which those beyond an even share count less, since blocks
+    // take items as they get done, and a fifth of an item for the last one's start, two fifths for 16-bit rows of an odd
+    // number of cells, whose ends take longer than other tiles; more for tiles with an x wall (the copying warp brings
+    // the wall slots), for the row ends of odd rows, and for rows that do not fill their tile.
+    //
+    // What is asked of the ratio is what no box of that set got slower with by more than 1 %; for rows of whole tiles,
+    // where the model is better, of another 600.
+    // F16SR 291 x 129 x 161: 180 us by pairs, 170 without; F32 37 x 157 x 177: 63 and 57; F16SR 128^3 58.2 and 59.7.
+    struct Model {
+        double plane, wall, odd, most;                    // this kernel
+        double start, l2, memory, row, unused, from, to;  // the others
+    };
+    static const Model models[5] = {{},
+                                    {1.80, 0.22, 0.10, 1.08, 2.9, 63100, 43800, 7.6, 0.83, 80e6, 120e6},
+                                    {1.60, 0.13, 0.20, 0.96, 5.6, 100200, 84100, 16.3, 1.29, 70e6, 130e6},
+                                    {1.58, 0.13, 0.15, 0.97, 6.8, 110400, 85600, 17.5, 1.21, 60e6, 130e6},
+                                    {1.81, 0.12, 0.25, 0.95, 8.6, 103800, 81700, 14.1, 1.17, 70e6, 120e6}};
+    const Model& m = models[storage];
+    const Split s = split(g, eb, sms);
+    const double cells = (double)g.nx * g.ny * g.nz, state = (double)Q * (double)g.S * eb;
+    const int vec = 16 / eb;
+    const double unused = (double)((g.nx + vec - 1) / vec * vec) / g.nx - 1.0;
+    const double memory = std::min(1.0, std::max(0.0, (state - m.from) / (m.to - m.from)));
+    const double separate = m.start + 2.0 * cells * ((1.0 - memory) / m.l2 +
+                                                     (memory * (1.0 + m.row / g.nx) + m.unused * unused) / m.memory);
+    const double chunks = (double)((g.nz + s.zc - 1) / s.zc);
+    const double even = (double)s.tiles * (g.nz + 2.0 * chunks) / sms;
+    double more = 1.0 + m.wall * std::min(1.0, 2.0 / (double)s.tiles_x);
+    if (g.nx % 2) more += m.odd / (double)s.tiles_x + (storage == 4 ? 0.06 : 0.0);
+    if (g.nx < kTX) more *= 1.15;
+    const double start = g.nx % 2 && eb == 2 ? 0.4 : 0.2;
+    const double pairs = 1.4 + m.plane * ((0.95 * even + 0.75 * ((double)s.planes - even)) * more + start * (s.zc + 2));
+    return pairs < (g.nx % kTX == 0 ? std::max(1.0, m.most) : m.most) * separate;
 }
 
 cudaError_t launch_pair_step(int storage, const void* in, void* out, const Grid& g, const Params& p, int lid_y,
