@@ -104,20 +104,15 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
 
 // Product with a constant, as two scalar multiplies: given a constant operand,
 // ptxas contracts mul.rn.f32x2 and the add or sub that follows into one fused
-// multiply-add (the scalar mul.rn.f32 it leaves alone), which changes the result.
-// The FP32 pipe takes as long for two scalar operations as for a paired one.
-// Products of two variables came out unfused, but nothing says that they must
-// where a sum follows: the squares of such a sum are fused multiply-adds of their
-// own, with -0, which are the rounded products (0.3 % of the FP32 kernel's time;
-// as scalar products 0.8 %).
+// multiply-add (the scalar mul.rn.f32 it leaves alone, and so it does products
+// of two variables), which changes the result.  The FP32 pipe takes as long for
+// two scalar operations as for a paired one.
 __device__ __forceinline__ F2 f2_scale(float c, F2 a)
 {
     float lo, hi;
     f2_split(a, lo, hi);
     return f2_make(__fmul_rn(c, lo), __fmul_rn(c, hi));
 }
-
-__device__ __forceinline__ F2 f2_square(F2 a) { return f2_fma(a, a, f2_both(-0.0f)); }
 
 // relax_pair (lbm_core.cuh) on two cells: the same operations in the same
 // order, except that P + (-3 s) is written P - 3 s, which is the same value.
@@ -154,7 +149,7 @@ __device__ __forceinline__ void collide_fluid2(F2* f, float inv_tau)
     r = r + f[16]; z = z + f[16];
     r = r + f[17]; z = z - f[17];
     r = r + f[18];
-    const F2 vel2 = f2_square(x) + f2_square(y) + f2_square(z);
+    const F2 vel2 = x * x + y * y + z * z;
     const F2 P = r - f2_scale(1.5f, vel2);
     constexpr float wa = 1.0f / 18.0f, wd = 1.0f / 36.0f;
     relax_pair2(f[0], f[1], wa, P, x, inv_tau);
