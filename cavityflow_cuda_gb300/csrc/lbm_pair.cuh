@@ -104,14 +104,27 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
 
 // Product with a constant, as two scalar multiplies: given a constant operand,
 // ptxas contracts mul.rn.f32x2 and the add or sub that follows into one fused
-// multiply-add (the scalar mul.rn.f32 it leaves alone, and so it does products
-// of two variables), which changes the result.  The FP32 pipe takes as long for
-// two scalar operations as for a paired one.
+// multiply-add, which changes the result; the scalar mul.rn.f32 it leaves alone.
+// The FP32 pipe takes as long for two scalar operations as for a paired one.
+// Paired products of two variables come out unfused so far, but nothing says that
+// they must where a paired sum follows, so such a sum is scalar (f2_sum3: 0.2 % of
+// the FP32 kernel's time; scalar products 0.8 %; fused multiply-adds with -0 in
+// place of the products do not do, ptxas makes products of them and contracts
+// those).
 __device__ __forceinline__ F2 f2_scale(float c, F2 a)
 {
     float lo, hi;
     f2_split(a, lo, hi);
     return f2_make(__fmul_rn(c, lo), __fmul_rn(c, hi));
+}
+
+__device__ __forceinline__ F2 f2_sum3(F2 a, F2 b, F2 c)
+{
+    float a0, a1, b0, b1, c0, c1;
+    f2_split(a, a0, a1);
+    f2_split(b, b0, b1);
+    f2_split(c, c0, c1);
+    return f2_make(__fadd_rn(__fadd_rn(a0, b0), c0), __fadd_rn(__fadd_rn(a1, b1), c1));
 }
 
 // relax_pair (lbm_core.cuh) on two cells: the same operations in the same
@@ -149,8 +162,7 @@ __device__ __forceinline__ void collide_fluid2(F2* f, float inv_tau)
     r = r + f[16]; z = z + f[16];
     r = r + f[17]; z = z - f[17];
     r = r + f[18];
-    const F2 vel2 = x * x + y * y + z * z;
-    const F2 P = r - f2_scale(1.5f, vel2);
+    const F2 P = r - f2_scale(1.5f, f2_sum3(x * x, y * y, z * z));
     constexpr float wa = 1.0f / 18.0f, wd = 1.0f / 36.0f;
     relax_pair2(f[0], f[1], wa, P, x, inv_tau);
     relax_pair2(f[2], f[3], wa, P, y, inv_tau);
