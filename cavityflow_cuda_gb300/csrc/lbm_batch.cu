@@ -321,10 +321,7 @@ int lbm_batch_get_info(const lbm_batch* b, lbm_batch_info* info)
                     (int64_t)((b->vb_cap[0] + b->vb_cap[1]) * (long long)sizeof(int));
     for (const lbm_solver* v : b->views) bytes += v->device_bytes;
     bytes += (int64_t)b->pack.bytes;
-    {
-        std::lock_guard<std::mutex> lock(b->second.mutex);
-        bytes += (int64_t)b->second.bytes;
-    }
+    bytes += (int64_t)b->second.bytes;
     info->device_bytes = bytes;
     return LBM_OK;
 }

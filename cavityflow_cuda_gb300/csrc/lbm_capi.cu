@@ -726,10 +726,7 @@ int lbm_get_info(const lbm_solver* s, lbm_info* info)
                                                                             : 0;
     info->row_pitch = s->g.P;
     info->slot_stride = s->g.S;
-    {
-        std::lock_guard<std::mutex> lock(s->second.mutex);
-        info->device_bytes = s->device_bytes + (int64_t)(s->pack.bytes + s->second.bytes);
-    }
+    info->device_bytes = s->device_bytes + (int64_t)(s->pack.bytes + s->second.bytes);
     info->lid_mode = s->lid_mode;
     info->moving_wall = s->p.wall_y > 0 ? 1 : 0;
     info->x1_column = s->g.xoff + 1;

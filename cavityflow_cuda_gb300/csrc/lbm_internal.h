@@ -48,10 +48,10 @@ private:
 // good, when an allocation of this library on that device finds too little
 // (lbm_memory.cu).
 struct SecondArray {
-    mutable std::mutex mutex;  // held to read or change what follows, and by a run until its launches are queued
+    std::mutex mutex;  // held to use or change what follows, and by a run until its launches are queued
     void* p = nullptr;
     void* image = nullptr;
-    size_t bytes = 0;          // of both
+    std::atomic<size_t> bytes{0};  // of both; read without the mutex, so that nobody waits for a run to know it
     bool refused = false;      // no memory for it, or given up
     int device = 0;
     bool listed = false;

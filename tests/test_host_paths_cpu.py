@@ -288,3 +288,29 @@ for n, count, rows in (((2, 900, 900), 4, (8, 6)), ((64, 64, 64), 76, (68, 68)),
         fake.fake_memory(1 << 40)
         assert run(b, 8) == 8
 """)
+
+
+def test_info_does_not_wait_for_a_run(child):
+    """A thread that watches another's run gets its answer while the launches are being queued."""
+    child("""
+for make in (solver, batch):
+    with make() as s:
+        run(s, 4)
+        reached, times = threading.Event(), []
+        def launch(name, args):
+            if b"pair_step" in name:
+                reached.set()
+                time.sleep(0.1)
+        watch(launch)
+        def look():
+            reached.wait()
+            t = time.perf_counter()
+            s.info()
+            times.append(time.perf_counter() - t)
+        t = threading.Thread(target=look)
+        t.start()
+        s.run(20)
+        t.join()
+        fake.fake_on_launch(None)
+        assert times[0] < 0.05, times
+""")
