@@ -107,6 +107,15 @@ int lbm_detail::default_batch_variant(int storage)
     }
 }
 
+// FP32 and FP64 keep two-cell and one-cell threads with direct windows (13) at every
+// size.  FP32, us a step in a replayed graph, variants 13 / 14 / 17 / 1 / 2 / 3: 16^3 1.65
+// / 1.89 / 1.93 / 3.60 / 3.20 / 2.12, 32^3 1.93 / 1.92 / 2.67 / 5.35 / 3.85 / 2.63, 48^3
+// 2.92 / 2.91 / 3.59 / 7.30 / 5.30 / 3.53, 64^3 5.31 / 5.40 / 6.28 / 8.87 / 8.66 / 6.16,
+// 80^3 9.28 / 9.35 / 10.9 / 16.1 / 15.1 / 10.9, 96^3 16.5 / 16.5 / 17.4 / 27.4 / 26.8 /
+// 18.5, 112^3 35.6 / 35.8 / 37.8 / 48.1 / 46.5 / 40.6 (1 and 2, four cells a thread, would
+// hold 64^3 in one wave).  FP64 with fused multiply-adds, 13 / 3: 24^3 7.5 / 12.4, 64^3
+// 73.7 / 74.2, 160^3 1081 / 1084.
+//
 // The 16-bit storages' 8- and 4-cell threads are long serial chains: on domains
 // that do not fill the chip with them fewer cells a thread are faster (us a step
 // in a replayed graph, F16SR: 32^3 variant 20 3.95, 6 2.67; 64^3 20 6.23, 6 5.67,

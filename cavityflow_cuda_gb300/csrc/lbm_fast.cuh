@@ -123,7 +123,9 @@ __device__ __forceinline__ B shfl_down_bits(B v, int d)
 // next step's waiting blocks would hold the places that spread its own over the
 // SMs.  Graph-replayed steps, before -> now (late / at once), us: 32^3 FP32 2.18
 // -> 1.96 / 2.87, 48^3 3.28 -> 2.95 / 3.36, 96^3 16.26 -> 16.34 / 16.00, 128^3
-// F16SR 29.83 -> 30.19 / 29.54.  Without the launch attribute (launch_step) both
+// F16SR 29.83 -> 30.19 / 29.54.  "Holds": 152 SMs with 512 threads each, what the
+// default shapes' 128 registers allow, as one border for all shapes: the two ways
+// differ much only far below it.  Without the launch attribute (launch_step) both
 // instructions do nothing.
 __device__ __forceinline__ void wait_previous_step() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_step() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

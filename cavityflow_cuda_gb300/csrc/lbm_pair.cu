@@ -133,8 +133,10 @@ cudaError_t launch_one(const void* in, void* out, const Grid& g, const Params& p
 // Tiles for a domain of a batch (FP32): the shape whose planes of the whole
 // domain take the least time.  A plane's time, fitted to 45 shapes from 12 x 32
 // to 128 x 3 (7 % off on average): its cells', and its rows', which a warp's
-// accesses straddle and the copies bring one by one.  Microseconds, GB300: 64 x 8
-// 2.5-2.8, 96 x 5 2.65, 48 x 10 2.5-2.7, 32 x 16 3.1-3.4, 14 x 32 3.8.
+// accesses straddle and the copies bring one by one.  Microseconds, GB300, whole
+// chip busy, boxes of one tile a row, all of whose tiles have both x walls: 64 x 8
+// 2.5-2.8 (2.1 in a large box), 96 x 5 2.65, 48 x 10 2.5-2.7, 32 x 16 3.1-3.4, 14 x
+// 32 3.8.
 template <class St>
 PairDims batch_dims(const Grid& g, double& plane)
 {
@@ -163,7 +165,7 @@ PairDims batch_dims(const Grid& g, double& plane)
 }
 
 template <class St>
-void plan_batch(int storage, const BatchDomain* doms, int count, PairBatchPlan& plan)
+void plan_batch(const BatchDomain* doms, int count, PairBatchPlan& plan)
 {
     constexpr int eb = (int)sizeof(typename St::bits);
     const int sms = sm_count();
@@ -291,7 +293,7 @@ cudaError_t launch_batch(const PairBatchPlan& plan, const void* image, bool back
 void plan_pair_batch(int storage, const BatchDomain* doms, int count, PairBatchPlan& plan)
 {
     plan = PairBatchPlan{};
-    if (storage == 1) plan_batch<F32>(storage, doms, count, plan);
+    if (storage == 1) plan_batch<F32>(doms, count, plan);
 }
 
 bool bind_pair_batch(int storage, const void* pool, const void* pool2, PairBatchPlan& plan)

@@ -32,20 +32,20 @@
 // rn.f32x2: the same IEEE operation on both cells, half the instructions).
 //
 // Measured on GB300 at 384^3 (ms a pair, separate kernels -> this one): FP32
-// 2.58 -> 1.49 (76.1 GLUP/s; 93 % of the copy bandwidth for the bytes it moves,
-// 1.11x its array in and 1.0x out), F16S 1.39 -> 1.05 and BF16S 1.38 -> 1.04 (109
-// GLUP/s), F16SR 1.41 -> 1.20 (94.4 GLUP/s; its dither is a fifth of its
-// instructions).  The 16-bit storages are bound by their instructions (56-63 %
-// of the issue slots used, with 25 warps a SM), not by memory.
+// 2.58 -> 1.49 (76.0 GLUP/s; 93 % of the copy bandwidth for the bytes it moves,
+// 1.11x its array in and 1.0x out), F16S 1.39 -> 1.07 and BF16S 1.38 -> 1.055 (107
+// GLUP/s), F16SR 1.41 -> 1.18 (95.7 GLUP/s; its dither is a fifth of its
+// instructions).  The 16-bit storages are bound by their instructions (55-62 %
+// of the issue slots used, with 24 warps a SM), not by memory.
 //
 // Batches (FP32): the items of all domains in one launch, the longest first, with
 // the tiles of each domain as they fit it best (batch_dims in lbm_pair.cu) and a
-// domain's layout and parameters in shared memory.  Same kernel, BATCH: a full
-// tile's plane takes 2.1 us instead of 1.9, 0.1 of it for 19 copies in place of
-// one and for addresses from shared memory, the rest for rows that start 8 bytes
-// past a sector.  GLUP/s, the separate kernels -> this one: 64 and 512 cavities
-// of 16 .. 96 cells an edge 35.8 -> 45.7 and 34.3 -> 47.9, 76 of 64^3 37 -> 51,
-// 610 of 32^3 34.7 -> 42.  The 16-bit storages stay with the separate kernels:
+// domain's layout and parameters in shared memory.  Same kernel, BATCH: with the
+// whole chip busy (384^3, a batch of one) a full tile's plane takes 2.1 us instead
+// of 1.9, 0.1 of it for 19 copies in place of one and for addresses from shared
+// memory, the rest for rows that start 8 bytes past a sector.  GLUP/s, the separate
+// kernels -> this one: 512 cavities of 16 .. 96 cells an edge 34.3 -> 50.4, 76 of
+// 64^3 37 -> 54, 610 of 32^3 34.7 -> 45.  The 16-bit storages stay with the separate kernels:
 // they move half the bytes and ran at 0.75 .. 1.0 of their speed here.
 #pragma once
 
@@ -310,6 +310,7 @@ struct Two<St, false> {
 template <class St, int TX, int TY, int NST, bool BATCH>
 struct PairShape {
     using bits = typename St::bits;
+    static_assert(!BATCH || sizeof(bits) == 4, "batches take two steps a pass in FP32 only");
     static constexpr int kAlign = 16 / (int)sizeof(bits);        // elements to a 16-byte boundary
     static constexpr int kUnit = 128 / (int)sizeof(bits);        // of a copy's destination
     static constexpr int kSlot = (TY + 2) * (TX + 2 * kAlign);
@@ -784,8 +785,10 @@ __device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& s
             const PairDims d = src.dims(item);
             const Grid& g = src.at(item).g;
             const int ry = tid / (d.tx / 2), px = tid % (d.tx / 2);
-            if (BATCH && !k16) SEP = d.tx / 2;
-            if (BATCH) W = d.w;
+            if (BATCH) {
+                SEP = d.tx / 2;
+                W = d.w;
+            }
             za = it.za;
             zb = it.zb;
             p = za - 1;
@@ -826,7 +829,8 @@ __device__ __forceinline__ void pair_beta(const PairSource<St, TX, TY, BATCH>& s
                 // their own are 1-8 % faster (FP32; 16-bit, for rows that do not fill their warp), but not with the
                 // dither of F16SR (2-4 % slower).
                 // Stores of the default policy: the neighbours' parts of a sector meet in L2. Streaming ones were slower:
-                // FP32 256^3 0.458 -> 0.450 ms a pair, batches of 64^3 0.750 -> 0.730 and of 40 x 72 x 50 0.531 -> 0.503.
+                // FP32 256^3 0.458 -> 0.450 ms a pair, batches of 64^3 0.750 -> 0.730 and of 40 x 72 x 50 0.531 -> 0.503
+                // when it was changed.
                 auto push = [&](auto cells) {
                     constexpr int kCells = decltype(cells)::value;  // 0: as vb says
                     static_for<0, Q>([&](auto kc) {

@@ -355,7 +355,7 @@ class CLbmSolverGB300:
         _check(self._lib.lbm_set_fast_variant(self._h, int(variant)))
 
     def autotune(self, pairs: int = 10):
-        """Time every launch variant on this domain and keep the fastest;
+        """Time every launch variant on this domain and keep the fastest for the steps taken one by one;
         the populations are restored.  Returns (best, ms per pair per variant)."""
         n = int(self._lib.lbm_fast_variant_count())
         ms = (C.c_float * n)()
@@ -506,6 +506,8 @@ class LbmBatch:
         _check(self._lib.lbm_batch_set_fast_variant(self._h, int(variant)))
 
     def autotune(self, pairs: int = 5):
+        """Time every register variant on the whole batch and keep the fastest for the steps taken one by one
+        (FP32 batches may take two steps a pass instead); (variant, ms per pair of each)."""
         ms = (C.c_float * self._lib.lbm_register_variant_count())()
         best = C.c_int32()
         _check(self._lib.lbm_batch_autotune(self._h, int(pairs), C.byref(best), ms))

@@ -276,7 +276,9 @@ int lbm_set_driven_cavity(lbm_solver* solver);
 
 /* ---- time steps -------------------------------------------------------------
  * Kernels are queued on `stream` and the call returns without waiting, as in
- * the reference. */
+ * the reference.  They are programmatic dependents of each other: a graph that
+ * the caller captures them into has programmatic edges (cudaGraphGetEdges wants
+ * an edge data array for such a graph), and replays as any other. */
 
 /* Whole domain.  Replaces CLbmSolverGPU<T>::simulationStepAlpha(stream)
  * (src/CLbmSolverGPU.cu:173-248). */
@@ -494,7 +496,8 @@ int lbm_batch_run(lbm_batch* batch, int64_t steps, void* stream);
  * lbm_set_fast_variant does. */
 int lbm_batch_set_fast_variant(lbm_batch* batch, int32_t variant);
 /* Times each register variant on the whole batch (`pairs` alpha/beta pairs,
- * CUDA events), keeps the fastest and restores the populations.  ms_per_pair
+ * CUDA events), keeps the fastest for the steps taken one by one and restores
+ * the populations.  ms_per_pair
  * (optional) receives lbm_register_variant_count() times, -1 for a variant
  * whose vectors are wider than the batch's packed rows (8 bytes).
  * Synchronous. */
