@@ -148,7 +148,9 @@ cudaError_t launch_step(Kernel kern, dim3 grid, int block, cudaStream_t st, size
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+    if (e != cudaSuccess) cudaGetLastError();  // the caller reports it; not the next launch, too
+    return e;
 }
 
 // The group of CPT cells a thread owns: group gi of row y of plane z.  An

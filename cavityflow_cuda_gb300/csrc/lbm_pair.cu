@@ -110,7 +110,10 @@ cudaError_t launch(const CUtensorMap& map, const PairCtx& one, const PairWork& w
     using S = PairShape<St, kTX, TY, NST, BATCH>;
     auto kern = pair_step<St, kTX, TY, NST, BATCH>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return e;
+    }
     const int grid = w.items < sms ? w.items : sms;
     return launch_step(kern, dim3((unsigned)grid), S::THREADS, st, S::SMEM, map, one, step_base, step_off, w, err);
 }

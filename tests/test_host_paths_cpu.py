@@ -314,3 +314,22 @@ for make in (solver, batch):
         fake.fake_on_launch(None)
         assert times[0] < 0.05, times
 """)
+
+
+@pytest.mark.parametrize("kernel", ["alpha_fast", "beta_fast_direct", "pair_step", "batch_step"])
+def test_failed_launch_is_reported_once(child, kernel):
+    """The runtime keeps a launch's error until it is asked for: the call that failed takes it away, so that the next
+    one does not report it again."""
+    child(f"kernel = {kernel!r}.encode()" + """
+with (batch() if kernel == b"batch_step" else solver()) as s:
+    v = s.domain(3) if kernel == b"batch_step" else s
+    if kernel != b"pair_step": s.set_fast_variant(s.info()["fast_variant"])
+    run(s, 1 if kernel == b"beta_fast_direct" else 4)
+    v.getDensities((1, 1, 1), (4, 4, 4))                        # the fields' memory is there
+    fake.fake_fail_launch(kernel, 1)
+    try: s.run(4); status = 0
+    except LbmError as e: status = e.status
+    assert status == 3
+    s.run(1)
+    v.getDensities((1, 1, 1), (4, 4, 4))
+""")
