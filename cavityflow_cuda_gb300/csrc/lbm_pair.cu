@@ -361,7 +361,7 @@ bool pair_step_pays(int storage, const Grid& g)
     const double even = (double)s.tiles * (g.nz + 2.0 * chunks) / sms;
     double more = 1.0 + m.wall * std::min(1.0, 2.0 / (double)s.tiles_x);
     if (g.nx % 2) more += m.odd / (double)s.tiles_x + (storage == 4 ? 0.06 : 0.0);
-    if (g.nx < kTX) more *= 1.15;
+    if (g.nx < kTX) more *= eb == 2 ? 1.25 : 1.15;  // 16 bits, 58 .. 62 wide: up to 1.2 times what the rest says
     const double start = g.nx % 2 && eb == 2 ? 0.4 : 0.2;
     const double pairs = 1.4 + m.plane * ((0.95 * even + 0.75 * ((double)s.planes - even)) * more + start * (s.zc + 2));
     return pairs < (g.nx % kTX == 0 ? std::max(1.0, m.most) : m.most) * separate;
