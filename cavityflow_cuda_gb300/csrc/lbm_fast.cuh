@@ -1046,7 +1046,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_step(typename St::bits* __r
     static_assert(kChunks <= BLOCK, "one thread per descriptor chunk");
     __shared__ BatchDomain desc[2];
     wait_previous_step();
-    allow_next_step();  // the next step's blocks take the places of those that run out of virtual blocks
+    // With many rounds over the grid the next step's blocks take the places of those that run out of virtual blocks; with
+    // few, they only get into the way of the last ones.  At once / at the end, us a step in a replayed graph: 16-bit
+    // 126 000 cells (0.4 rounds) 7.36 / 5.80, 434 000 (1.6) 10.2 / 8.82, 1.39 M (5) 22.95 / 21.20, 2.77 M (9.5) 45.9 / 45.2,
+    // 4.18 M (14.6) 75.0 / 76.2; FP32 218 000 cells 8.05 / 7.20, 959 000 (6) 23.35 / 22.12, 2.06 M (13) 61.0 / 60.6, 4.13 M
+    // 116.9 / 118.0.
+    if (vblocks >= 12ll * gridDim.x) allow_next_step();
     const long long stride = gridDim.x;
     long long vb = blockIdx.x;
     if (vb >= vblocks) return;
@@ -1077,6 +1082,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_step(typename St::bits* __r
         else if constexpr (kBeta == 1) beta_cells_blk<St, CPT, BLOCK>(dd, g, inv_tau, lid_u, lid_y, wall_y, c, ds);
         else beta_cells<St, CPT>(dd, g, inv_tau, lid_u, lid_y, wall_y, c, ds);
     }
+    allow_next_step();  // does nothing the second time
 }
 
 template <class St, int VARIANT, bool kAlpha>
