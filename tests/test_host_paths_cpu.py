@@ -271,13 +271,15 @@ for make in (solver, batch):
 
 
 def test_batch_without_room_for_row_padding_keeps_its_narrow_rows(child):
-    """Rows are padded to what two steps a pass need only where the padded pool fits."""
+    """Rows are padded to what two steps a pass need only where those pay and the padded pool fits."""
     child("""
 def pool(b, n, count):
     return count * 19 * 4 * b.domain(0).info()["slot_stride"]
-for n, count, rows in (((2, 900, 900), 4, (8, 6)), ((64, 64, 64), 76, (68, 68)), ((65, 64, 64), 76, (72, 70))):
+for n, count, rows in (((2, 900, 900), 4, (6, 6)), ((64, 64, 64), 76, (68, 68)), ((65, 64, 64), 76, (72, 70))):
     with batch(n, count) as b:
         assert b.domain(0).info()["row_pitch"] == rows[0], b.domain(0).info()["row_pitch"]
+        assert run(b, 8) == (8 if rows[0] == 6 else 4)
+    with batch(n, count) as b:
         wide, rest = pool(b, n, count), b.info()["device_bytes"] - pool(b, n, count)
     if rows[0] == rows[1]: continue
     assert wide * rows[1] // rows[0] + rest < wide - 1
