@@ -225,7 +225,10 @@ static int batch_create_unguarded(const lbm_domain_spec* domains, int32_t count,
     } free_if_thrown{b};
     b->storage = storage;
     b->device = device;
-    b->variant = default_batch_variant(storage);
+    long long cells = 0;
+    for (int i = 0; i < count; ++i)
+        cells += (long long)domains[i].size[0] * domains[i].size[1] * domains[i].size[2];
+    b->variant = default_batch_variant(storage, cells);
     add_second_array(b->second, device);
     auto bail = [&](int r) { free_batch(b); return r; };
 

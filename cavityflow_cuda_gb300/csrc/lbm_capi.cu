@@ -90,20 +90,23 @@ constexpr int kGraphPairs = 32;  // alpha/beta pairs per captured graph
 }  // namespace
 
 // Batch and server rows are packed for 8-byte vectors (kPackedX1Align), so
-// their variants use 8-byte (or narrower) vectors in both kernels.  On the
-// seeded workload (ms a pair of 64 / 512 cavities): FP32 the direct beta windows
-// in four-warp blocks (variant 14: 0.728 / 5.32; 13, two warps: 0.755 / 5.51; 17,
-// eight: 0.736 / 5.28, and behind 14 on 8 cavities), the 16-bit storages the
+// their variants use 8-byte (or narrower) vectors in both kernels.  FP32 and
+// FP64: the direct beta windows, in four-warp blocks (14) or, for batches that
+// leave a part of the chip idle, two-warp ones (13).  The 16-bit storages: the
 // packed beta at <= 128 registers (22: the batch kernel's own state spills the
-// 102-register shape), FP64 the warp exchange (3: 6.71 of 64; 13: 6.98).
-int lbm_detail::default_batch_variant(int storage)
+// 102-register shape).  us a step in a replayed graph, boxes of uneven size, FP32
+// 13 / 14: 27 000 cells 2.95 / 3.45, 99 000 4.33 / 4.33, 366 000 9.59 / 9.36, 2.0 M
+// 61.3 / 58.4, 6.3 M 191 / 178; FP64 13 / 14 / 3 (the warp exchange in eight-warp
+// blocks): 28 000 13.0 / 14.3 / 19.1, 151 000 49.0 / 53.9 / 66.3, 885 000 251 / 252 /
+// 264, 2.5 M 675 / 666 / 687, 8.2 M 2185 / 2158 / 2225.
+int lbm_detail::default_batch_variant(int storage, long long cells)
 {
     switch (storage) {
     case LBM_STORAGE_F16S:
     case LBM_STORAGE_BF16S:
     case LBM_STORAGE_F16SR: return 22;
-    case LBM_STORAGE_F64: return 3;
-    default: return 14;
+    case LBM_STORAGE_F64: return cells < 1100000 ? 13 : 14;
+    default: return cells < 350000 ? 13 : 14;
     }
 }
 

@@ -128,8 +128,9 @@ int elem_bytes(int storage);
 int value_bytes(int storage);
 // Default register variant of a domain.
 int default_variant(int storage, const lbm::Grid& g);
-// Default register variant of the batch kernel (many small domains).
-int default_batch_variant(int storage);
+// Default register variant of the batch kernel for domains of that many interior
+// cells together.
+int default_batch_variant(int storage, long long cells);
 // Creates a solver; with `external_dd` its populations live there (a batch
 // pool) and are initialised but never freed by the solver.
 // x1_align, pitch_align: 32, 0 (the default layout) or those of batch pools'

@@ -369,7 +369,7 @@ int lbm_server_create(const lbm_server_config* cfg, lbm_server** out)
     s->cfg = *cfg;
     s->cfg.max_round_steps &= ~1;
     s->variant = cfg->fast_variant > 0 && cfg->fast_variant <= lbm::kRegisterVariants ? cfg->fast_variant - 1
-                                                                                       : default_batch_variant(cfg->storage);
+                                                                                       : default_batch_variant(cfg->storage, 1ll << 40);
     const int32_t probe[3] = {8, 8, 8};  // any box: the packed rows' alignment does not depend on its size
     if (!lbm::fast_variant_fits(cfg->storage, s->variant, request_grid(probe, cfg->storage))) {
         delete s;

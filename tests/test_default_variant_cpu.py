@@ -21,3 +21,13 @@ for n, want in {CASES!r}:
     with solver(n, {storage!r}) as s:
         assert s.info()["fast_variant"] == want, (n, s.info()["fast_variant"])
 """)
+
+
+@pytest.mark.parametrize("storage,n,count,variant", [("f32", (20, 20, 20), 10, 13), ("f32", (64, 64, 64), 2, 14),
+                                                     ("f64", (64, 64, 64), 4, 13), ("f64", (64, 64, 64), 5, 14),
+                                                     ("f16sr", (20, 20, 20), 10, 22), ("f16sr", (64, 64, 64), 9, 22)])
+def test_default_variant_of_batches(child, storage, n, count, variant):  # noqa: F811
+    child(f"""
+with batch({n}, {count}, {storage!r}) as b:
+    assert b.info()["fast_variant"] == {variant}, b.info()["fast_variant"]
+""")

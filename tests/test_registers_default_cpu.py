@@ -22,8 +22,12 @@ BUDGETS = [
     ("fast_f32.cu", "batch_step<lbm::F32, 2, 128, 4, false, 2>", 128, 0),
     ("fast_f64.cu", "alpha_fast<lbm::F64, 1, 64, 8>", 128, 0),
     ("fast_f64.cu", "beta_fast_direct<lbm::F64, 1, 64, 8>", 128, 0),
-    ("fast_f64.cu", "batch_step<lbm::F64, 1, 256, 2, true, 0>", 128, 0),
-    ("fast_f64.cu", "batch_step<lbm::F64, 1, 256, 2, false, 0>", 128, 84),
+    ("fast_f32.cu", "batch_step<lbm::F32, 2, 64, 8, true, 2>", 128, 48),
+    ("fast_f32.cu", "batch_step<lbm::F32, 2, 64, 8, false, 2>", 128, 0),
+    ("fast_f64.cu", "batch_step<lbm::F64, 1, 64, 8, true, 2>", 128, 0),
+    ("fast_f64.cu", "batch_step<lbm::F64, 1, 64, 8, false, 2>", 128, 0),
+    ("fast_f64.cu", "batch_step<lbm::F64, 1, 128, 4, true, 2>", 128, 0),
+    ("fast_f64.cu", "batch_step<lbm::F64, 1, 128, 4, false, 2>", 128, 0),
     ("fast_f16sr.cu", "alpha_fast<lbm::F16SR, 2, 256, 2>", 128, 0),
     ("fast_f16sr.cu", "beta_fast<lbm::F16SR, 2, 256, 2>", 128, 0),
     ("fast_f16sr.cu", "alpha_fast<lbm::F16SR, 4, 64, 8>", 128, 0),
