@@ -123,6 +123,7 @@ private:
 struct lbm_server {
     lbm_server_config cfg{};
     int variant = 0;
+    bool own_variant = false;  // the caller's; otherwise each table's default
     char* arena = nullptr;
     size_t arena_bytes = 0;
     Arena alloc;
@@ -225,9 +226,15 @@ int admit(lbm_server* s)
     return LBM_OK;
 }
 
-// Packs the given requests into the device table for `variant`.
+// Packs the given requests into the device table for `variant`, the default one
+// for so many cells unless the caller chose.
 int upload_table(lbm_server* s, const std::vector<Request*>& reqs, long long (&vblocks)[2])
 {
+    if (!s->own_variant) {
+        long long cells = 0;
+        for (const Request* r : reqs) cells += (long long)r->g.nx * r->g.ny * r->g.nz;
+        s->variant = default_batch_variant(s->cfg.storage, cells);
+    }
     s->table.resize(reqs.size());
     long long next[2] = {0, 0};
     for (size_t i = 0; i < reqs.size(); ++i) {
@@ -368,8 +375,8 @@ int lbm_server_create(const lbm_server_config* cfg, lbm_server** out)
     if (!s) return fail(LBM_ERR_OUT_OF_MEMORY, "host allocation failed");
     s->cfg = *cfg;
     s->cfg.max_round_steps &= ~1;
-    s->variant = cfg->fast_variant > 0 && cfg->fast_variant <= lbm::kRegisterVariants ? cfg->fast_variant - 1
-                                                                                       : default_batch_variant(cfg->storage, 1ll << 40);
+    s->own_variant = cfg->fast_variant > 0 && cfg->fast_variant <= lbm::kRegisterVariants;
+    s->variant = s->own_variant ? cfg->fast_variant - 1 : default_batch_variant(cfg->storage, 1ll << 40);
     const int32_t probe[3] = {8, 8, 8};  // any box: the packed rows' alignment does not depend on its size
     if (!lbm::fast_variant_fits(cfg->storage, s->variant, request_grid(probe, cfg->storage))) {
         delete s;
