@@ -116,7 +116,7 @@ inline Grid make_grid(int nx, int ny, int nz, int elem_bytes, int x1_align = 32,
 
 // Alignment of x = 1 in the rows of batch and server boxes (see above).
 constexpr int kPackedX1Align = 8;
-// Rows of an FP32 batch: whole multiples of the 16 bytes that a tensor copy
+// Rows of an FP32 batch that takes two steps a pass: whole multiples of the 16 bytes that a tensor copy
 // (lbm_pair.cuh) needs of its strides.  With 32, 64 and 128 bytes the pair kernel took
 // 2-5 %, 6-23 % and 10-36 % longer.  The other storages' batches run without it.
 inline int batch_pitch_align(int storage) { return storage == 1 ? 16 : 0; }
